@@ -48,7 +48,7 @@ DEFAULT_BUCKETS = [
 
 # candidate settings per stage of the search (coordinate descent)
 _MODES = [{"force_mode": -1}, {"force_mode": 0}, {"force_mode": 1}, {"force_mode": 2}]
-_SCATTER = [{"scatter": s} for s in range(9)]
+_PART_FILL = [{"part_fill_pct": p} for p in (50, 60, 70)]
 _SMEM = [{"smem_bytes": b, "smem_fill_pct": f} for b in (48 << 10, 96 << 10, 160 << 10) for f in (50, 70)]
 _LOAD = [{"load_factor_pct": p} for p in (40, 50, 70)]
 
@@ -272,14 +272,14 @@ def _time(keys, reqs, tuning: Dict[str, int], steps: int) -> float:
 
 def tune_bucket(rows: int, groups: int, steps: int = 5, verbose: bool = False) -> Tuple[Dict[str, int], Dict]:
     """Coordinate descent: mode, then (for the chosen mode) the partition
-    launch shape or the shared-memory table, then the load factor."""
+    table fill or the shared-memory table, then the load factor."""
     keys, reqs = _workload(rows, groups)
     log = {}
     best: Dict[str, int] = {}
     best_ms = _time(keys, reqs, best, steps)
     log["default"] = best_ms
-    for stage in (_MODES, _SCATTER, _SMEM, _LOAD):
-        if stage is _SCATTER and best.get("force_mode", -1) not in (-1, 2):
+    for stage in (_MODES, _PART_FILL, _SMEM, _LOAD):
+        if stage is _PART_FILL and best.get("force_mode", -1) not in (-1, 2):
             continue
         if stage is _SMEM and best.get("force_mode", -1) not in (-1, 1):
             continue

@@ -18,8 +18,7 @@
 #include "gb_engine.h"
 #include "gb_kernels.cuh"
 #include "gb_partition.cuh"
-#include "gb_scatter.h"
-#include "gb_sorted.h"
+#include "gb_record.h"
 
 namespace gb {
 
@@ -717,24 +716,10 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
     }
   }
   int64_t smem_max = opt.smem_max_groups >= 0 ? opt.smem_max_groups : (int64_t)sfill;
-  // partitioned pass 2.  Per-row variant: as many slots as fit ~220 KB (any
-  // count), one more for the all-ones key.  Sorted-chunk variants: the slots
-  // that fit beside the chunk's sorted stage and the two per-slot count arrays.
-  bool any_val_null = false;
-  for (int v = 0; v < P.num_vals; ++v) any_val_null |= P.vals[v].mask != nullptr;
-  const bool p2_sorted = opt.pass2 != 1 && opt.pass2 != 4;
-  const int p2_rows = part_sorted_rows(opt.pass2, P.num_vals);  // rows per sorted chunk
-  int scap2;
-  if (p2_sorted) {
-    const size_t budget = (size_t)std::min(227 * 1024, dev.smem_optin) - 4096;
-    const size_t fixed = part_sorted_smem(P, 0, p2_rows, any_val_null);
-    const size_t per_slot = (size_t)P.slot_bytes + 8;
-    scap2 = budget > fixed + 256 + 2 * per_slot ? (int)((budget - fixed - 256) / per_slot) - 1 : 0;
-    while (scap2 > 0 && part_sorted_smem(P, scap2, p2_rows, any_val_null) > budget) --scap2;
-    scap2 = std::min(scap2, 65000);  // slot indices are 16-bit in the sorted stage
-  } else {
-    scap2 = std::max(0, std::min(220 * 1024, dev.smem_optin - 8192) / P.slot_bytes - 1);
-  }
+  // partitioned pass 2: as many slots as fit ~220 KB (any count), one more for
+  // the all-ones key
+  const int scap_rec = std::max(0, std::min(220 * 1024, dev.smem_optin - 8192) / (P.slot_bytes + 4) - 1) & ~3;  // with tags
+  const int scap2 = std::max(0, std::min(220 * 1024, dev.smem_optin - 8192) / P.slot_bytes - 1);
   const int sfill2 = std::max(1, (int)(scap2 * 0.8));
   bool part_ok = !P.has_arg && !P.need_second_pass && P.num_vals <= 8 && scap2 >= 256;
   for (int v = 0; v < P.num_vals; ++v) part_ok = part_ok && P.vals[v].basic;
@@ -742,15 +727,20 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
     uint8_t op = P.accs[a].op;
     if (op >= OP_PROD_I64 && op <= OP_PROD_F64) part_ok = false;
   }
-  // partitions: enough for ~70% table fill, at most 8192 (the scatter's
-  // per-tile partition arrays take 16 B each in shared memory); beyond
-  // ~85% of that capacity the shared tables would spill most groups and
-  // the global table is faster
+  // partitions: enough for the wanted table fill.  Up to 2048 they are a
+  // multiple of the SM count, so that pass 2 ends in whole waves and a tile's
+  // runs are no shorter than the tables need; a partition then holds 8 or more
+  // of the 2^14 hash buckets, give or take one.  Above that a power of two,
+  // whose partitions hold equally many buckets, at most 8192 (the scatter
+  // keeps 12 B per partition in shared memory); beyond ~85% of that capacity
+  // the shared tables would spill most groups and the global table is faster.
   constexpr int kMaxParts = 8192;
   int nparts = 0;
   if (part_ok) {
-    double per = scap2 * opt.part_fill;
-    nparts = (int)std::min<uint64_t>(kMaxParts, std::max<uint64_t>(2, next_pow2((uint64_t)std::ceil(est / per))));
+    const int64_t want = std::max<int64_t>(2, (int64_t)std::ceil((double)est / (scap_rec * opt.part_fill)));
+    const int64_t whole = (want + dev.sms - 1) / dev.sms * dev.sms;
+    const int64_t tight = (int64_t)std::ceil((double)est / (scap_rec * std::max(opt.part_fill, 0.78)));
+    nparts = (int)(whole <= 2048 ? whole : (int64_t)std::min<uint64_t>(kMaxParts, next_pow2((uint64_t)tight)));
   }
   const bool part_fits = (double)est <= 0.85 * (double)kMaxParts * sfill2;
   int mode;
@@ -770,9 +760,8 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
       nsamp = (int64_t)buckets.size();
       exact_buckets = false;
     }
-    int lg = 0;
-    while ((1 << lg) < nparts) ++lg;
-    int per_bucket = kBucketBits - lg;
+    constexpr int64_t kBuckets = 1 << kBucketBits;
+    auto first_bucket = [&](int64_t p) { return (p * kBuckets + nparts - 1) / nparts; };  // see part_of
     pbase.resize(nparts);
     pend.resize(nparts);
     prows.resize(nparts);
@@ -781,7 +770,7 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
     for (auto b : buckets) samp += b;
     for (int p = 0; p < nparts; ++p) {
       double c = 0;
-      for (int b = p << per_bucket; b < ((p + 1) << per_bucket); ++b) c += buckets[b];
+      for (int64_t b = first_bucket(p); b < first_bucket(p + 1); ++b) c += buckets[b];
       int64_t capp;
       if (exact_buckets) {
         capp = (int64_t)c;
@@ -833,64 +822,24 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
       std::memcpy(st3 + 2 * nparts, pbase.data(), 8 * nparts);
       ck(cudaMemcpyAsync(d_base, st3, 24 * (size_t)nparts, cudaMemcpyHostToDevice, stream), "h2d");
     }
-    PartArgs A;
+    RecSpec rec;
+    if (!record_layout(P, rec)) throw Error(ERR_LOGIC, "internal error: plan without a record layout");
+    RecArgs A;
     std::memset(&A, 0, sizeof(A));
     A.nparts = nparts;
-    int lg = 0;
-    while ((1 << lg) < nparts) ++lg;
-    A.shift = 64 - lg;
-    A.base = d_base;
     A.end = d_end;
     A.cursor = d_cur;
-    A.keys = (uint64_t*)S.get((size_t)total * 8 * P.key_words);
-    bool any_null = false;
-    for (int v = 0; v < P.num_vals; ++v) {
-      A.vals[v] = S.get((size_t)total * P.vals[v].width);
-      any_null |= P.vals[v].mask != nullptr;
-    }
-    A.bits = any_null ? (uint8_t*)S.get((size_t)total) : nullptr;
+    A.recs = (uint64_t*)S.get((size_t)total * 8 * rec.words);
     A.counters = counters;
     mark("partition scratch");
     if (opt.profile) ck(cudaEventRecord(events()[0], stream), "event");
-    {
-      auto launch = [&](auto kern, int nt, int rpt) {
-        size_t psmem = part_scatter_smem(P.key_words, nt * rpt, nparts);
-        allow_max_smem((const void*)kern);
-        int grid = grid_for((const void*)kern, nt, psmem, 0);
-        kern<<<grid, nt, psmem, stream>>>(P, A);
-      };
-      const bool kw1 = P.key_words == 1;
-      // 7 (the default): tiles staged by bulk copies when every column allows
-      // it; 8: the same with 2048-row tiles, two CTAs per SM
-      std::vector<uint8_t> spec(part_scatter_spec_bytes());
-      const size_t bsm = opt.scatter >= 7
-                           ? part_scatter_bulk_plan(P, nparts, dev.smem_optin, spec.data(), opt.scatter == 8)
-                           : 0;
-      if (bsm) launch_part_scatter_bulk(P, A, spec.data(), bsm, stream);
-      else switch (opt.scatter) {
-        case 1: kw1 ? launch(k_part_scatter<1, 16, 256, 3>, 256, 16) : launch(k_part_scatter<2, 16, 256, 3>, 256, 16); break;
-        case 2: kw1 ? launch(k_part_scatter<1, 16, 512, 2>, 512, 16) : launch(k_part_scatter<2, 16, 512, 2>, 512, 16); break;
-        case 3: kw1 ? launch(k_part_scatter<1, 8, 1024, 1>, 1024, 8) : launch(k_part_scatter<2, 8, 1024, 1>, 1024, 8); break;
-        case 4: kw1 ? launch(k_part_scatter<1, 8, 512, 3>, 512, 8) : launch(k_part_scatter<2, 8, 512, 3>, 512, 8); break;
-        case 5: kw1 ? launch(k_part_scatter<1, 4, 1024, 2, false>, 1024, 4) : launch(k_part_scatter<2, 4, 1024, 2, false>, 1024, 4); break;
-        case 6: kw1 ? launch(k_part_scatter<1, 8, 256, 4>, 256, 8) : launch(k_part_scatter<2, 8, 256, 4>, 256, 8); break;
-        default: kw1 ? launch(k_part_scatter<1, 8, 512, 3, false>, 512, 8) : launch(k_part_scatter<2, 8, 512, 2, false>, 512, 8); break;
-      }
-    }
+    if (!launch_rec_scatter(P, A, rec, dev.smem_optin, stream))
+      throw Error(ERR_LOGIC, "internal error: no launch shape for the partition pass");
     ++st.kernels;
     ck(cudaGetLastError(), "partition launch");
     if (opt.profile) ck(cudaEventRecord(events()[4], stream), "event");
 
     // ---- pass 2: per-partition shared-memory aggregation ----
-    Plan P2 = P;
-    P2.packed_keys = A.keys;
-    for (int v = 0; v < P.num_vals; ++v) {
-      P2.vals[v].data = A.vals[v];
-      P2.vals[v].mask = nullptr;
-      P2.vals[v].offset = 0;
-      P2.vals[v].bits = A.bits;
-      P2.vals[v].bit = v;
-    }
     // pass-2 work: one item per partition, except that a partition holding
     // far more rows than the average (a heavy key) is cut into row ranges
     // handled by several CTAs, each merging its table into the global table
@@ -933,6 +882,12 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
     }
     PartItem* d_items = (PartItem*)S.get(sizeof(PartItem) * items.size());
     ck(cudaMemcpyAsync(d_items, items.data(), sizeof(PartItem) * items.size(), cudaMemcpyHostToDevice, stream), "h2d");
+    // a table four times the groups expected in a partition costs no probes
+    // and less to reset than all of shared memory (a caller's estimate may be
+    // far off: it gets the whole table)
+    const int scap_p = exact_buckets ? (int)std::min<int64_t>(scap_rec, 4 * (est / nparts) + 256) & ~3
+                                     : scap_rec;
+    const int sfill_p = std::max(1, (int)(scap_p * 0.9));
     // groups expected to miss their partition's shared table, plus those of
     // split partitions, go to the global spill table
     const double expect_spill = std::max(0.0, (double)est - 0.85 * (double)nparts * sfill2);
@@ -953,68 +908,25 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
       ck(cudaMemsetAsync(counters + 6, 0, 8 * 4, stream), "memset");
       G = TableRef{T, spill_cap - 1, P.slot_bytes, P.key_words, counters};
       DenseRef D{dense, dcap, (unsigned long long*)(counters + 10), counters + 6};
-      // shared table plus the all-ones key's slot (sorted variants: plus the
-      // count arrays and the chunk's sorted stage)
-      size_t sm2 = p2_sorted ? part_sorted_smem(P, scap2, p2_rows, any_val_null)
-                             : (size_t)(scap2 + 1) * P.slot_bytes;
       // items of split (heavy) partitions first, with rows of one slot
       // combined per warp before their shared update; then the rest
-      auto launch2 = [&](auto kern, int nt, int first, int count, unsigned int* work) {
+      auto launch2 = [&](int first, int count, unsigned int* work, bool wagg) {
         if (count <= 0) return;
-        PartArgs Ai = A;
+        RecArgs Ai = A;
         Ai.items = d_items + first;
         Ai.nitems = count;
         Ai.work = work;
-        allow_max_smem((const void*)kern);
-        int grid = grid_for((const void*)kern, nt, sm2, 0);
-        grid = std::min(grid, count);
-        kern<<<grid, nt, sm2, stream>>>(P2, Ai, G, D, scap2, sfill2, tmpl);
+        (P.key_words == 1 ? launch_rec_aggregate1 : launch_rec_aggregate2)(P, Ai, rec, G, D, scap_p, sfill_p, tmpl, wagg,
+                                                                           stream);
         ++st.kernels;
       };
-      auto launch_s = [&](int first, int count, unsigned int* work, bool wagg) {
-        if (count <= 0) return;
-        PartArgs Ai = A;
-        Ai.items = d_items + first;
-        Ai.nitems = count;
-        Ai.work = work;
-        launch_part_sorted(opt.pass2, P2, Ai, G, D, scap2, sfill2, tmpl, sm2, wagg, stream);
-        ++st.kernels;
-      };
-      const bool few = P.num_vals <= 4;
-      const int nrest = (int)items.size() - nwagg;
-      if (p2_sorted) {
-        launch_s(0, nwagg, counters + 8, true);
-        launch_s(nwagg, nrest, counters + 9, false);
-      } else if (opt.pass2 == 4 && few) {  // 512 threads x 2 rows
-        if (P.key_words == 1) {
-          launch2(k_part_aggregate<1, 2, 512, 4, true>, 512, 0, nwagg, counters + 8);
-          launch2(k_part_aggregate<1, 2, 512, 4, false>, 512, nwagg, nrest, counters + 9);
-        } else {
-          launch2(k_part_aggregate<2, 2, 512, 4, true>, 512, 0, nwagg, counters + 8);
-          launch2(k_part_aggregate<2, 2, 512, 4, false>, 512, nwagg, nrest, counters + 9);
-        }
-      } else if (P.key_words == 1) {
-        if (few) {
-          launch2(k_part_aggregate<1, 1, 1024, 4, true>, 1024, 0, nwagg, counters + 8);
-          launch2(k_part_aggregate<1, 1, 1024, 4, false>, 1024, nwagg, nrest, counters + 9);
-        } else {
-          launch2(k_part_aggregate<1, 1, 1024, 8, true>, 1024, 0, nwagg, counters + 8);
-          launch2(k_part_aggregate<1, 1, 1024, 8, false>, 1024, nwagg, nrest, counters + 9);
-        }
-      } else {
-        if (few) {
-          launch2(k_part_aggregate<2, 1, 1024, 4, true>, 1024, 0, nwagg, counters + 8);
-          launch2(k_part_aggregate<2, 1, 1024, 4, false>, 1024, nwagg, nrest, counters + 9);
-        } else {
-          launch2(k_part_aggregate<2, 1, 1024, 8, true>, 1024, 0, nwagg, counters + 8);
-          launch2(k_part_aggregate<2, 1, 1024, 8, false>, 1024, nwagg, nrest, counters + 9);
-        }
-      }
+      launch2(0, nwagg, counters + 8, true);
+      launch2(nwagg, (int)items.size() - nwagg, counters + 9, false);
       if (opt.profile) ck(cudaEventRecord(events()[1], stream), "event");
       // rows listed as not fitting their partition's table (none when the
       // sample sized the partitions well): one grid-stride launch that reads
       // the list length on the device
-      k_part_spill<false><<<dev.sms * 2, 256, 0, stream>>>(P2, G, A);
+      launch_rec_spill(P, A, rec, G, dev.sms * 2, stream);
       k_finish_count<<<1, 1, 0, stream>>>(P, G);
       st.kernels += 3;
       ck(cudaGetLastError(), "partition aggregate launch");
@@ -1037,7 +949,6 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
         st.scatter_ms = ms1;
       }
       mark("partition passes (synced)");
-      if (host[14]) throw Error(ERR_CUDA, "partition pass: a bulk copy did not complete in time");
       if (host[5]) break;  // a region overflowed: fall back to the global table
       if (host[1] == 0 && host[6] == 0 && host[13] == 0) {
         done = true;
@@ -1120,7 +1031,7 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
                                   : launch_raw(k_part_aggregate<1, 1, 1024, 8, true, true>);
         else few ? launch_raw(k_part_aggregate<2, 1, 1024, 4, true, true>)
                  : launch_raw(k_part_aggregate<2, 1, 1024, 8, true, true>);
-        k_part_spill<true><<<dev.sms * 2, 256, 0, stream>>>(P, G, A);
+        k_part_spill<<<dev.sms * 2, 256, 0, stream>>>(P, G, A);
         st.kernels += 2;
       } else if (mode == 1) {
         size_t sm = (size_t)scap * P.slot_bytes;
@@ -1229,7 +1140,6 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
     ck(cudaStreamSynchronize(stream), "compact sync");
     mark("compaction (synced)");
     if (deferred) {
-      if (host[14]) throw Error(ERR_CUDA, "partition pass: a bulk copy did not complete in time");
       // an overflow anywhere (a table, a region, the dense slots, a spill
       // list): redo the call with checks after every stage
       const bool again = host[1] || chost[1] || (mode == 2 && (host[5] || host[6] || host[13])) ||

@@ -77,9 +77,9 @@ struct Options {
   int64_t groups_hint = -1;    // caller's group-count estimate (-1: sample)
   int force_mode = -1;         // -1 auto, 0 global only, 1 smem stage
   int profile = 0;             // time kernels with CUDA events
-  int scatter = 7;             // partitioned pass 1: 7 bulk-copy tiles where the columns allow (else 0), 0-6 launch shapes of the per-thread scatter
-  double part_fill = 0.7;      // partitioned mode: expected groups per partition / shared-table slots (sets the partition count)
-  int pass2 = 1;               // partitioned pass 2: 1 per-row shared reductions, 0/2 sorted chunks 512x4, 3 sorted 256x8
+  int scatter = 7;             // accepted 0-8: earlier launch shapes of partitioned pass 1, which now picks its own
+  double part_fill = 0.6;      // partitioned mode: expected groups per partition / shared-table slots (sets the partition count)
+  int pass2 = 1;               // accepted 0-4: earlier forms of partitioned pass 2, which now has one
   int wagg_pct = 125;          // partitioned pass 2: warp-combined updates for partitions above this % of the average rows
   uint32_t set_mask = 0;       // OPT_* bits of the fields a caller set explicitly
   // internal: 0 reads every outcome (group counts, overflow flags, null

@@ -5,21 +5,19 @@
 // SM-free table op on B200), far below HBM bandwidth.  This path trades one
 // extra write+read of the rows for atomics that stay in shared memory:
 //
-//   k_part_scatter    pass 1: pack each row's key, take the top bits of its
-//                     hash as partition id, and scatter key words, value bits
-//                     and a validity byte into that partition's region.  One
-//                     global atomic per (tile, partition) reserves space.
-//   k_part_aggregate  pass 2: one CTA at a time owns a work item -- a
-//                     partition, or a row range of a heavy partition -- and
-//                     aggregates it in a shared-memory table; its groups are
+//   k_rec_scatter     pass 1 (gb_record.cuh): pack each row's key, take its
+//                     hash bucket as partition, and store the row as one record
+//                     in that partition's region.
+//   k_rec_aggregate   pass 2 (gb_record.cuh): one CTA at a time owns a work item
+//                     -- a partition, or a record range of a heavy partition --
+//                     and aggregates it in a shared-memory table; its groups are
 //                     then copied out as dense slots (or merged into a global
 //                     spill table for split partitions and partitions that did
-//                     not fit).  Items of split partitions combine the rows of
-//                     one slot per warp before the shared update.  The same
-//                     kernel over row ranges of the caller's own columns is
-//                     the shared-stage mode for groups that fit one CTA.
+//                     not fit).
+//   k_part_aggregate  the shared-stage mode for groups that fit one CTA: row
+//                     ranges of the caller's own columns through such a table.
 //   k_part_spill      applies the rows listed as not fitting their table to
-//                     the global spill table.
+//                     the global table.
 #pragma once
 #include <cub/block/block_scan.cuh>
 
@@ -64,276 +62,6 @@ struct DenseRef {
 __device__ __forceinline__ void prefetch_l2(const void* p)
 {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-
-// Pass 1.  Each CTA takes tiles of RPT*NT rows.  A tile's rows are counting-
-// sorted by partition in shared memory, so every (tile, partition) run leaves
-// as one contiguous write of ~tile/nparts rows instead of scattered stores:
-//   A  keys loaded (all RPT per thread at once), partition id = top hash bits,
-//      rank within the tile's partition from a shared histogram;
-//   B  one global reservation per (tile, partition) on the region cursor,
-//      exclusive scan of the histogram; per partition, `delta` maps a sorted
-//      position to its global row and `send` bounds the rows that fit;
-//   C  keys, then each value column, then the validity bytes are stored into
-//      the stage at their sorted position and written out in sorted order
-//      (consecutive threads, consecutive rows of a run).  The next column's
-//      loads are issued before the current column's write-out.
-// Shared memory: stage[tile * 8] | psort u16[tile] | hist u32[nparts] |
-//                send u32[nparts] | delta i64[nparts]
-template <int KW, int RPT, int NT, int MINB, bool PF = true>
-__global__ void __launch_bounds__(NT, MINB) k_part_scatter(const __grid_constant__ Plan P,
-                                                         const __grid_constant__ PartArgs A)
-{
-  constexpr int TILE = RPT * NT;
-  static_assert(TILE <= 65536, "sorted positions are 16-bit");
-  extern __shared__ __align__(16) uint8_t sh[];
-  uint8_t* stage = sh;
-  uint16_t* psort = (uint16_t*)(sh + (size_t)TILE * 8);
-  unsigned int* hist = (unsigned int*)(psort + TILE);
-  unsigned int* send = hist + A.nparts;
-  long long* delta = (long long*)(send + A.nparts + (A.nparts & 1));
-  using Scan = cub::BlockScan<unsigned, NT>;
-  __shared__ typename Scan::TempStorage scan_tmp;
-  __shared__ unsigned int s_valid;
-  const int64_t n = P.num_rows;
-  const bool any_bits = A.bits != nullptr;
-  const int nv = P.num_vals;
-  const int per = (A.nparts + NT - 1) / NT;  // partitions per thread in the scan
-  for (int64_t t0 = (int64_t)blockIdx.x * TILE; t0 < n; t0 += (int64_t)gridDim.x * TILE) {
-    const int cnt = (int)(n - t0 < (int64_t)TILE ? n - t0 : (int64_t)TILE);
-    for (int i = threadIdx.x; i < A.nparts; i += NT) hist[i] = 0;
-    __syncthreads();
-    // A
-    uint32_t pr[RPT];  // partition << 16 | rank, later partition << 16 | sorted position
-    const bool plain_key =
-      P.num_keys == 1 && !P.keys[0].mask && P.keys[0].width == 8 && P.keys[0].cat != CAT_F64;
-    const unsigned long long* kd = (const unsigned long long*)P.keys[0].data + P.keys[0].offset;
-    if (plain_key) {
-      // one plain 64-bit key: its bits are the key word
-      uint64_t k0[RPT];
-#pragma unroll
-      for (int k = 0; k < RPT; ++k) {
-        const int i = k * NT + threadIdx.x;
-        k0[k] = i < cnt ? __ldg(kd + t0 + i) : 0;
-      }
-#pragma unroll
-      for (int k = 0; k < RPT; ++k) {
-        const int i = k * NT + threadIdx.x;
-        pr[k] = 0xFFFFFFFFu;
-        if (i < cnt) {
-          const unsigned p = (unsigned)(hash_key(k0[k], 0, 1) >> A.shift);
-          pr[k] = (p << 16) | atomicAdd(&hist[p], 1u);
-        }
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < RPT; ++k) {
-        const int i = k * NT + threadIdx.x;
-        pr[k] = 0xFFFFFFFFu;
-        uint64_t w0 = 0, w1 = 0;
-        if (i < cnt && pack_key(P, t0 + i, w0, w1)) {
-          const unsigned p = (unsigned)(hash_key(w0, w1, KW) >> A.shift);
-          pr[k] = (p << 16) | atomicAdd(&hist[p], 1u);
-        }
-      }
-    }
-    __syncthreads();
-    // B: reservations (independent atomics, issued before their results are
-    // used), then the scan
-    unsigned mine = 0;
-    for (int q0 = threadIdx.x * per; q0 < min(A.nparts, (threadIdx.x + 1) * per); q0 += 4) {
-      unsigned h[4];
-      unsigned long long g[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int q = q0 + j;
-        h[j] = (j < per && q < min(A.nparts, (threadIdx.x + 1) * per)) ? hist[q] : 0u;
-        g[j] = h[j] ? atomicAdd(&A.cursor[q], (unsigned long long)h[j]) : 0ull;
-        mine += h[j];
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int q = q0 + j;
-        if (!h[j]) continue;
-        const long long room = (long long)A.end[q] - (long long)g[j];
-        if ((long long)h[j] > room) atomicOr(A.counters + 5, 1u);
-        delta[q] = (long long)g[j];                      // minus the scan offset below
-        send[q] = room <= 0 ? 0u : (unsigned)min((long long)h[j], room);  // plus the offset below
-      }
-    }
-    unsigned off, total;
-    Scan(scan_tmp).ExclusiveSum(mine, off, total);
-    for (int q = threadIdx.x * per; q < min(A.nparts, (threadIdx.x + 1) * per); ++q) {
-      const unsigned h = hist[q];
-      if (h) {
-        delta[q] -= (long long)off;
-        send[q] += off;
-      }
-      hist[q] = off;  // partition start in the sorted tile
-      off += h;
-    }
-    if (threadIdx.x == 0) s_valid = total;
-    __syncthreads();
-    const int nvalid = (int)s_valid;
-    // C: sorted positions; keys (read again: the tile was just loaded, so
-    // they come from cache) through the stage
-#pragma unroll
-    for (int k = 0; k < RPT; ++k) {
-      if (pr[k] == 0xFFFFFFFFu) continue;
-      const unsigned p = pr[k] >> 16;
-      const unsigned s = hist[p] + (pr[k] & 0xFFFFu);
-      pr[k] = (p << 16) | s;
-      psort[s] = (uint16_t)p;
-    }
-    // two-word keys go through the 8-byte stage one word at a time (word 1
-    // waits in registers), which halves the stage and lets two CTAs share an SM
-    uint64_t kw1[KW == 2 ? RPT : 1];
-    if (plain_key) {
-      uint64_t k0[RPT];
-#pragma unroll
-      for (int k = 0; k < RPT; ++k) k0[k] = pr[k] != 0xFFFFFFFFu ? __ldg(kd + t0 + k * NT + threadIdx.x) : 0;
-#pragma unroll
-      for (int k = 0; k < RPT; ++k)
-        if (pr[k] != 0xFFFFFFFFu) ((uint64_t*)stage)[pr[k] & 0xFFFFu] = k0[k];
-    } else {
-#pragma unroll
-      for (int k = 0; k < RPT; ++k) {
-        if (pr[k] == 0xFFFFFFFFu) continue;
-        uint64_t w0 = 0, w1 = 0;
-        pack_key(P, t0 + k * NT + threadIdx.x, w0, w1);
-        ((uint64_t*)stage)[pr[k] & 0xFFFFu] = w0;
-        if (KW == 2) kw1[k] = w1;
-      }
-    }
-    // first value column's loads in flight with the key write-out
-    uint64_t x[RPT];
-    auto load_col = [&](int v) {
-      const ValCol& c = P.vals[v];
-#pragma unroll
-      for (int k = 0; k < RPT; ++k) {
-        const int i = k * NT + threadIdx.x;
-        x[k] = pr[k] != 0xFFFFFFFFu ? load_bits(c.data, t0 + i + c.offset, c.width) : 0;
-      }
-    };
-    // a column of at most 4 bytes shares its round with the validity bytes
-    // (value at +0 and validity at +4 of an 8-byte stage slot), saving the
-    // validity bytes' own round; it goes last, once every column's validity
-    // bit is known
-    int vn = -1;
-    if (any_bits)
-      for (int v = 0; v < nv; ++v)
-        if (P.vals[v].width <= 4) vn = v;
-    auto col_at = [&](int vi) { return vn < 0 || vi < vn ? vi : (vi == nv - 1 ? vn : vi + 1); };
-    if (PF && nv > 0) load_col(col_at(0));
-    __syncthreads();
-    for (int s = threadIdx.x; s < nvalid; s += NT) {
-      const unsigned p = psort[s];
-      if ((unsigned)s >= send[p]) continue;
-      const int64_t g = delta[p] + s;
-      A.keys[KW * g] = ((const uint64_t*)stage)[s];
-    }
-    if (KW == 2) {
-      __syncthreads();
-#pragma unroll
-      for (int k = 0; k < RPT; ++k)
-        if (pr[k] != 0xFFFFFFFFu) ((uint64_t*)stage)[pr[k] & 0xFFFFu] = kw1[k];
-      __syncthreads();
-      for (int s = threadIdx.x; s < nvalid; s += NT) {
-        const unsigned p = psort[s];
-        if ((unsigned)s >= send[p]) continue;
-        A.keys[2 * (delta[p] + s) + 1] = ((const uint64_t*)stage)[s];
-      }
-    }
-    // validity bytes of this thread's rows, four to a register
-    uint32_t vb[(RPT + 3) / 4];
-#pragma unroll
-    for (int k = 0; k < (RPT + 3) / 4; ++k) vb[k] = 0;
-#pragma unroll 1
-    for (int vi = 0; vi < nv; ++vi) {
-      const int v = col_at(vi);
-      const ValCol& c = P.vals[v];
-      if (any_bits) {
-#pragma unroll
-        for (int k = 0; k < RPT; ++k)
-          if (pr[k] != 0xFFFFFFFFu && (!c.mask || bit_valid(c.mask, t0 + k * NT + threadIdx.x + c.offset)))
-            vb[k >> 2] |= 1u << (v + 8 * (k & 3));
-      }
-      if (!PF) load_col(v);
-      __syncthreads();  // the previous write-out has read the stage
-      void* dst = A.vals[v];
-      if (v == vn) {
-#pragma unroll
-        for (int k = 0; k < RPT; ++k)
-          if (pr[k] != 0xFFFFFFFFu) {
-            const unsigned s = pr[k] & 0xFFFFu;
-            ((uint32_t*)stage)[2 * s] = (uint32_t)x[k];
-            stage[8 * s + 4] = (uint8_t)(vb[k >> 2] >> (8 * (k & 3)));
-          }
-        __syncthreads();
-        for (int s = threadIdx.x; s < nvalid; s += NT) {
-          const unsigned p = psort[s];
-          if ((unsigned)s >= send[p]) continue;
-          const int64_t g = delta[p] + s;
-          const uint32_t w = ((const uint32_t*)stage)[2 * s];
-          if (c.width == 4) ((uint32_t*)dst)[g] = w;
-          else if (c.width == 2) ((uint16_t*)dst)[g] = (uint16_t)w;
-          else ((uint8_t*)dst)[g] = (uint8_t)w;
-          A.bits[g] = stage[8 * s + 4];
-        }
-        continue;
-      }
-#pragma unroll
-      for (int k = 0; k < RPT; ++k)
-        if (pr[k] != 0xFFFFFFFFu) store_width(stage, pr[k] & 0xFFFFu, c.width, x[k]);
-      __syncthreads();
-      if (PF && vi + 1 < nv) load_col(col_at(vi + 1));
-      switch (c.width) {
-        case 8:
-          for (int s = threadIdx.x; s < nvalid; s += NT) {
-            const unsigned p = psort[s];
-            if ((unsigned)s < send[p]) ((uint64_t*)dst)[delta[p] + s] = ((const uint64_t*)stage)[s];
-          }
-          break;
-        case 4:
-          for (int s = threadIdx.x; s < nvalid; s += NT) {
-            const unsigned p = psort[s];
-            if ((unsigned)s < send[p]) ((uint32_t*)dst)[delta[p] + s] = ((const uint32_t*)stage)[s];
-          }
-          break;
-        case 2:
-          for (int s = threadIdx.x; s < nvalid; s += NT) {
-            const unsigned p = psort[s];
-            if ((unsigned)s < send[p]) ((uint16_t*)dst)[delta[p] + s] = ((const uint16_t*)stage)[s];
-          }
-          break;
-        default:
-          for (int s = threadIdx.x; s < nvalid; s += NT) {
-            const unsigned p = psort[s];
-            if ((unsigned)s < send[p]) ((uint8_t*)dst)[delta[p] + s] = stage[s];
-          }
-          break;
-      }
-    }
-    if (any_bits && vn < 0) {
-      __syncthreads();
-#pragma unroll
-      for (int k = 0; k < RPT; ++k)
-        if (pr[k] != 0xFFFFFFFFu) stage[pr[k] & 0xFFFFu] = (uint8_t)(vb[k >> 2] >> (8 * (k & 3)));
-      __syncthreads();
-      for (int s = threadIdx.x; s < nvalid; s += NT) {
-        const unsigned p = psort[s];
-        if ((unsigned)s < send[p]) A.bits[delta[p] + s] = stage[s];
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// shared-memory bytes of k_part_scatter for a tile of `tile` rows
-inline size_t part_scatter_smem(int kw, int tile, int nparts)
-{
-  (void)kw;
-  return (size_t)tile * 8 + (size_t)tile * 2 + (size_t)nparts * 8 + 8 + (size_t)nparts * 8;
 }
 
 // Shared-memory find-or-insert; null when the key does not fit (table at its
@@ -483,9 +211,8 @@ __device__ __forceinline__ void smax_u32(uint32_t a, uint32_t v) { if (v > sld_u
 // loop carries no call into the generic update code.  The list count lives in
 // counters[12]; counters[13] is set when the list itself overflowed (the host
 // then re-runs pass 2 with a longer list).
-template <bool RAW = false>
-__global__ void __launch_bounds__(256) k_part_spill(const __grid_constant__ Plan P2, TableRef G,
-                                                    const __grid_constant__ PartArgs A)
+static __global__ void __launch_bounds__(256) k_part_spill(const __grid_constant__ Plan P2, TableRef G,
+                                                           const __grid_constant__ PartArgs A)
 {
   __shared__ unsigned int s_new;
   if (threadIdx.x == 0) s_new = 0;
@@ -494,12 +221,7 @@ __global__ void __launch_bounds__(256) k_part_spill(const __grid_constant__ Plan
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
     const int64_t r = A.spill_rows[i];
     uint64_t w0, w1;
-    if (RAW) {
-      if (!pack_key(P2, r, w0, w1)) continue;  // not listed: null keys are skipped first
-    } else {
-      w0 = P2.packed_keys[r * P2.key_words];
-      w1 = P2.key_words == 2 ? P2.packed_keys[r * 2 + 1] : 0;
-    }
+    if (!pack_key(P2, r, w0, w1)) continue;  // not listed: null keys are skipped first
     const uint64_t h = hash_key(w0, w1, P2.key_words);
     const int64_t gi = global_slot(P2, G, w0, w1, h, &s_new);
     if (gi < 0) {
@@ -517,12 +239,12 @@ __global__ void __launch_bounds__(256) k_part_spill(const __grid_constant__ Plan
 // slots plus, for one-word keys, the slot of the all-ones key).  Returns the
 // item index (>= nitems: no work left).
 template <int NT>
-__device__ __forceinline__ int p2_claim(const PartArgs& A, uint8_t* smem, int scap, int nw,
+__device__ __forceinline__ int p2_claim(unsigned int* work, uint8_t* smem, int scap, int nw,
                                         const SlotTemplate& tmpl, int* s_part, unsigned int* s_used,
                                         unsigned int* s_spill)
 {
   if (threadIdx.x == 0) {
-    *s_part = (int)atomicAdd(A.work, 1u);
+    *s_part = (int)atomicAdd(work, 1u);
     *s_used = 0;
     *s_spill = 0;
   }
@@ -779,7 +501,7 @@ __global__ void __launch_bounds__(NT, 1) k_part_aggregate(const __grid_constant_
     }
   }
   for (;;) {
-    const int it = p2_claim<NT>(A, smem, scap + (KW == 1), nw, tmpl, &s_part, &s_used, &s_spill);
+    const int it = p2_claim<NT>(A.work, smem, scap + (KW == 1), nw, tmpl, &s_part, &s_used, &s_spill);
     if (it >= A.nitems) break;
     const PartItem item = A.items[it];
     const int64_t b = item.begin;

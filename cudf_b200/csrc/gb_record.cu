@@ -1,0 +1,139 @@
+// gb_record.cu -- record layout and the launchers of pass 1 and the spill pass
+// (gb_record.cuh), in their own compilation unit.
+#include <algorithm>
+#include <cstring>
+
+#include "gb_engine.h"
+#include "gb_record.cuh"
+
+namespace gb {
+
+bool record_layout(const Plan& P, RecSpec& S)
+{
+  std::memset(&S, 0, sizeof(S));
+  if (P.num_vals > kMaxRecCols) return false;
+  int key_bits = 0;
+  for (int k = 0; k < P.num_keys; ++k) {
+    const KeyCol& c = P.keys[k];
+    key_bits = std::max(key_bits, 64 * c.word + c.shift + 8 * c.width);
+    if (c.has_null_bit) key_bits = std::max(key_bits, 64 * c.null_word + c.null_shift + 1);
+  }
+  const int key_bytes = P.key_words == 2 ? 16 : key_bits <= 32 ? 4 : 8;
+  S.keymask = key_bytes == 4 ? 0xFFFFFFFFull : ~0ull;
+  for (int v = 0; v < P.num_vals; ++v) S.has_bits |= P.vals[v].mask != nullptr;
+  // widest columns first, each in the first free place aligned to its width
+  int order[kMaxRecCols];
+  for (int v = 0; v < P.num_vals; ++v) order[v] = v;
+  std::stable_sort(order, order + P.num_vals, [&](int a, int b) { return P.vals[a].width > P.vals[b].width; });
+  int at[kMaxRecCols];
+  const int sizes[] = {2, 4, 6, 8, 12};
+  for (int words : sizes) {
+    bool used[8 * kMaxRecWords] = {};
+    for (int i = 0; i < key_bytes; ++i) used[i] = true;
+    if (S.has_bits) used[8 * words - 1] = true;
+    bool fits = key_bytes <= 8 * words;
+    for (int j = 0; j < P.num_vals && fits; ++j) {
+      const int w = P.vals[order[j]].width;
+      int o = 0;
+      for (; o + w <= 8 * words; o += w) {
+        bool free = true;
+        for (int i = 0; i < w; ++i) free = free && !used[o + i];
+        if (free) break;
+      }
+      if (o + w > 8 * words) { fits = false; break; }
+      for (int i = 0; i < w; ++i) used[o + i] = true;
+      at[order[j]] = o;
+    }
+    if (fits) { S.words = words; break; }
+  }
+  if (S.words == 0) return false;
+  std::stable_sort(order, order + P.num_vals, [&](int a, int b) { return at[a] < at[b]; });
+  S.ncols = P.num_vals;
+  int word = P.key_words - 1;
+  for (int j = 0; j < P.num_vals; ++j) {
+    const ValCol& c = P.vals[order[j]];
+    S.src_col[j] = order[j];
+    S.off[j] = at[order[j]];
+    const bool nothing = c.sum_off < 0 && c.min_off < 0 && c.max_off < 0 && c.sq_off < 0;
+    const uint32_t kind = nothing            ? RK_NONE
+                          : c.cat == CAT_F64 ? RK_F64
+                          : c.cat == CAT_F32 ? RK_F32
+                          : c.width == 8     ? RK_W64
+                          : c.cat == CAT_SIGNED ? RK_S32 : RK_Z32;
+    const uint32_t flags = (c.cat == CAT_SIGNED ? RF_SIGNED : 0) | (c.cat == CAT_BOOL ? RF_BOOL : 0) |
+                           (c.sum_op == OP_SUM_I32 ? RF_SUM32 : 0);
+    const uint32_t ext = c.width < 4 ? 32 - 8 * c.width : 0;
+    const uint32_t shift = 8 * (S.off[j] % 8), adv = S.off[j] / 8 - word;
+    word = S.off[j] / 8;
+    S.col[j] = RecCol{{(uint32_t)(uint16_t)c.sum_off | (uint32_t)(uint16_t)c.min_off << 16,
+                       (uint32_t)(uint16_t)c.max_off | (uint32_t)(uint16_t)c.sq_off << 16,
+                       (uint32_t)(uint16_t)c.nulls_off | kind << 16 | shift << 24,
+                       adv | ext << 8 | flags << 16 | (uint32_t)order[j] << 24}};
+  }
+  for (int v = 0; v < P.num_vals; ++v) {
+    if (P.vals[v].mask) {
+      S.mask_col[S.nmask] = v;
+      S.mask_bit[S.nmask++] = (uint8_t)v;
+    } else {
+      S.vb_const |= (uint8_t)(1u << v);
+    }
+  }
+  const KeyCol& k = P.keys[0];
+  S.key8 = P.num_keys == 1 && k.width == 8 && k.mask == nullptr && k.word == 0 && k.shift == 0 &&
+           (k.cat == CAT_SIGNED || k.cat == CAT_UNSIGNED);
+  return true;
+}
+
+namespace {
+template <int KW, int NT, int RPT, int MINB>
+bool launch(const Plan& P, const RecArgs& A, const RecSpec& S, int smem_optin, cudaStream_t stream)
+{
+  const size_t T = (size_t)NT * RPT;
+  const size_t smem = T * S.words * 8 + (size_t)A.nparts * 8 + (size_t)S.nmask * (T / 32 + 1) * 4;
+  if ((smem + 2048) * MINB > (size_t)smem_optin) return false;
+  const int64_t ntiles = (P.num_rows + (int64_t)T - 1) / (int64_t)T;
+  auto go = [&](auto kern) {
+    allow_max_smem((const void*)kern);
+    const int grid = (int)std::min<int64_t>(grid_for((const void*)kern, NT, smem, MINB), ntiles);
+    kern<<<grid, NT, smem, stream>>>(P, A, S);
+  };
+  // reservations in flight across phase C while their results fit registers
+  const int per = (A.nparts + NT - 1) / NT;
+  if (per <= 2) go(k_rec_scatter<KW, NT, RPT, MINB, 2>);
+  else if (per <= 8) go(k_rec_scatter<KW, NT, RPT, MINB, 8>);
+  else go(k_rec_scatter<KW, NT, RPT, MINB, 1>);
+  return true;
+}
+template <int KW>
+bool pick(const Plan& P, const RecArgs& A, const RecSpec& S, int o, cudaStream_t s)
+{
+  // Two CTAs per SM on the largest tile of which two fit, so that one loads
+  // while the other reserves or writes.  With less than two rows per partition
+  // in such a tile (thousands of partitions) one CTA on a tile as large as
+  // shared memory instead: 40M 16-byte rows over 4096 partitions take 0.68 ms
+  // against 0.85, 100M 32-byte rows over 740 partitions 1.63 against 1.58.
+  if (A.nparts > 6144 / S.words) {  // two CTAs of T rows hold about 12,288 words each
+    if constexpr (KW == 1)
+      if (launch<KW, 1024, 8, 1>(P, A, S, o, s)) return true;
+    if (launch<KW, 1024, 6, 1>(P, A, S, o, s) || launch<KW, 1024, 5, 1>(P, A, S, o, s)) return true;
+  }
+  if constexpr (KW == 1)
+    if (launch<KW, 512, 8, 2>(P, A, S, o, s)) return true;
+  return launch<KW, 512, 6, 2>(P, A, S, o, s) || launch<KW, 512, 5, 2>(P, A, S, o, s) ||
+         launch<KW, 512, 4, 2>(P, A, S, o, s) || launch<KW, 512, 3, 2>(P, A, S, o, s) ||
+         launch<KW, 512, 2, 2>(P, A, S, o, s) || launch<KW, 512, 1, 2>(P, A, S, o, s);
+}
+}  // namespace
+
+bool launch_rec_scatter(const Plan& P, const RecArgs& A, const RecSpec& S, int smem_optin, cudaStream_t stream)
+{
+  return P.key_words == 1 ? pick<1>(P, A, S, smem_optin, stream) : pick<2>(P, A, S, smem_optin, stream);
+}
+
+void launch_rec_spill(const Plan& P, const RecArgs& A, const RecSpec& S, const TableRef& G, int grid,
+                      cudaStream_t stream)
+{
+  k_rec_spill<<<grid, 256, 0, stream>>>(P, G, A, S);
+}
+
+}  // namespace gb

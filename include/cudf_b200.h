@@ -140,19 +140,13 @@ typedef struct gb_tuning {
   int32_t force_mode;
   int64_t groups_hint;      /* caller's estimate of the number of groups (skips sampling) */
   int32_t profile;          /* 1: time the aggregation and compaction kernels with CUDA events */
-  int32_t scatter;          /* partitioned pass 1: 7 (default) tiles of 4096 (or 2048) rows staged in
-                               shared memory by bulk copies when every column allows it (16-byte
-                               aligned rows), else 0; 0-6 the per-thread launch shapes, threads x
-                               rows per thread: 0 512x8, 1 256x16, 2 512x16, 3 1024x8, 4 512x8 with
-                               the next column's loads issued early, 5 1024x4, 6 256x8; 8 as 7 with
-                               2048-row tiles, two CTAs per SM */
-  int32_t pass2;            /* partitioned pass 2: 1 per-row shared reductions (default); 0 (or 2)
-                               chunks counting-sorted by slot, 512 threads x 4 rows; 3 sorted,
-                               256 threads x 8 rows; 4 per-row, 512 threads x 2 rows (plans of
-                               up to four value columns, else as 1) */
+  int32_t scatter;          /* 0-8, accepted and without effect: partitioned pass 1 picks its launch
+                               shape by the record size and the partition count */
+  int32_t pass2;            /* 0-4, accepted and without effect: partitioned pass 2 has one form */
   int32_t part_fill_pct;    /* partitioned mode: expected groups per partition as a percentage of
-                               the pass-2 shared table's slots (default 70; sets the partition
-                               count, a power of two) */
+                               the pass-2 shared table's slots (default 60; sets the partition
+                               count: a multiple of the SM count up to 2048, above that a power of
+                               two at up to 78%) */
   int32_t wagg_pct;         /* partitioned pass 2: a partition holding more rows than this percentage
                                of the average partition (a heavy key) has the rows of one slot
                                combined per warp before each shared update (default 125; 0: every

@@ -1,0 +1,90 @@
+"""The partitioned path's row records against the oracle: every record size,
+key widths, column offsets, row counts around the tile edges, and values at the
+ends of their types."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from parity import run_both
+
+pytestmark = pytest.mark.gpu
+
+# value columns per schema: records of 16, 32, 48, 64 and 96 bytes
+SCHEMAS = {
+    16: ["i32", "f32"],
+    32: ["f64", "i64", "u8", "i16"],
+    48: ["f64", "i64", "f64", "f32", "bool"],
+    64: ["f64", "i64", "f64", "i64", "f32", "i32", "i8"],
+    96: ["f64", "i64", "f64", "i64", "f64", "i64", "f64", "u64"],
+}
+DTYPE = {"i8": np.int8, "u8": np.uint8, "i16": np.int16, "i32": np.int32, "i64": np.int64, "u64": np.uint64,
+         "f32": np.float32, "f64": np.float64, "bool": np.uint8}
+
+
+def _values(rng, kind, n):
+    dt = DTYPE[kind]
+    if kind == "bool":
+        return rng.integers(0, 2, n).astype(dt)
+    if kind in ("f32", "f64"):
+        v = rng.normal(size=n).astype(dt)
+        v[rng.random(n) < 0.002] = np.nan
+        v[rng.random(n) < 0.001] = -0.0
+        return v
+    info = np.iinfo(dt)
+    v = rng.integers(max(info.min, -1000), min(info.max, 1000), n, endpoint=True).astype(dt)
+    ends = rng.random(n)
+    v[ends < 0.001] = info.min
+    v[ends > 0.999] = info.max
+    return v
+
+
+def _column(cb, rng, arr, nullable, offset, type_id=None):
+    valid = rng.random(arr.shape[0]) > 0.15 if nullable else None
+    c = cb.Column.from_numpy(arr, valid, type_id)
+    return cb.Column(c.type_id, c.data, c.mask, size=arr.shape[0] - offset, offset=offset)
+
+
+@pytest.mark.parametrize("offset", [0, 3])
+@pytest.mark.parametrize("nullable", [False, True])
+@pytest.mark.parametrize("key", ["i32", "i64", "i64+i32", "i8+i16"])
+@pytest.mark.parametrize("size", sorted(SCHEMAS))
+@pytest.mark.parametrize("n", [1, 511, 3073, 40_961, 300_007])
+def test_record_shapes(n, size, key, nullable, offset):
+    import cudf_b200 as cb
+    from cudf_b200 import aggregation as agg
+    rng = np.random.default_rng(n * 7 + size)
+    rows = n + offset
+    ids = rng.integers(0, max(1, n // 3), rows)
+    parts = {"i32": [ids.astype(np.int32)], "i64": [ids * 1_000_003 - 5],
+             "i64+i32": [ids * 1_000_003, (ids % 7).astype(np.int32)],
+             "i8+i16": [(ids % 100).astype(np.int8), (ids % 3000).astype(np.int16)]}[key]
+    two = "+" in key
+    keys = [_column(cb, rng, k, two, offset) for k in parts]
+    # integral sums and sums of squares of values near the ends wrap alike; a
+    # float column with huge values would only loosen its own bound
+    reqs = []
+    for j, kind in enumerate(SCHEMAS[size]):
+        aggs = [agg.sum(), agg.min(), agg.max(), agg.count()]
+        if j == 0:
+            aggs += [agg.mean(), agg.sum_of_squares()]
+        c = _column(cb, rng, _values(rng, kind, rows), nullable, offset, O.BOOL8 if kind == "bool" else None)
+        reqs.append((c, aggs))
+    run_both(keys, reqs, include_null_keys=two, tuning={"force_mode": 2})
+
+
+@pytest.mark.parametrize("groups", [5_000, 900_000, 2_500_000])
+def test_table_fill_and_partition_counts(groups):
+    """Few, hundreds and thousands of partitions with tables near their fill
+    limit; every group has about two rows."""
+    import cudf_b200 as cb
+    from cudf_b200 import aggregation as agg
+    rng = np.random.default_rng(groups)
+    n = max(2 * groups, 1_100_000) + 13
+    key = rng.integers(0, groups, n).astype(np.int64) * 2_654_435_761
+    v = rng.integers(-10**9, 10**9, n)
+    f = rng.normal(size=n)
+    wide = [agg.sum(), agg.min(), agg.max(), agg.mean()]
+    gb, *_ = run_both([cb.Column.from_numpy(key)],
+                      [(cb.Column.from_numpy(v, rng.random(n) > 0.1), wide), (cb.Column.from_numpy(f), wide)],
+                      tuning={"force_mode": 2, "part_fill_pct": 85})
+    assert gb.stats()["mode"] == 2
