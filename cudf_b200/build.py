@@ -16,7 +16,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT, "libcudf_b200.so")
 
-SOURCES = ["gb_engine.cu", "gb_record.cu", "gb_record_agg1.cu", "gb_record_agg2.cu", "gb_capi.cu", "gb_noalloc.cu",
+SOURCES = ["gb_engine.cu", "gb_record.cu", "gb_record_agg1.cu", "gb_record_agg2.cu", "gb_stage.cu", "gb_capi.cu", "gb_noalloc.cu",
            "gb_batch.cu", "gb_server.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

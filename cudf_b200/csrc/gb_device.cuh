@@ -102,6 +102,83 @@ __device__ __forceinline__ uint64_t hash_key(uint64_t w0, uint64_t w1, int words
   return words == 1 ? fmix64(w0) : fmix64(w0 ^ fmix64(w1 + 0x9E3779B97F4A7C15ull));
 }
 
+// Folds one key column's loaded bits of R rows into their key words.  What a
+// column needs (normalising, a shift, its word, null flags) is the same for
+// all rows, so it is decided once per column.  valid[r] bit 0: not null;
+// live[r] is cleared for rows that EXCLUDE drops.
+template <int KW, int R>
+__device__ __forceinline__ void fold_key_column(const Plan& P, const KeyCol& c, uint64_t (&x)[R], const uint32_t (&valid)[R],
+                                                uint64_t (&k0)[R], uint64_t (&k1)[R], bool (&live)[R])
+{
+  if (c.cat == CAT_F32 || c.cat == CAT_F64 || c.cat == CAT_BOOL) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) x[r] = norm_key_bits(c, x[r]);
+  }
+  if (c.shift) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) x[r] <<= c.shift;
+  }
+  if (c.mask) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (!(valid[r] & 1u)) x[r] = 0;
+    if (!P.include_nulls) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) live[r] = live[r] && (valid[r] & 1u);
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const uint64_t flag = (uint64_t)(~valid[r] & 1u) << c.null_shift;
+        if (KW == 1 || c.null_word == 0) k0[r] |= flag;
+        else k1[r] |= flag;
+      }
+    }
+  }
+  if (KW == 1 || c.word == 0) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) k0[r] |= x[r];
+  } else {
+#pragma unroll
+    for (int r = 0; r < R; ++r) k1[r] |= x[r];
+  }
+}
+
+// Packed keys of the R rows first + 32 r of a thread, column by column with
+// the loads of all rows in flight together (as pack_key, per row).  live[r] is
+// cleared for rows that take no part.
+template <int KW, int R>
+__device__ __forceinline__ void pack_rows(const Plan& P, int64_t first, uint64_t (&k0)[R], uint64_t (&k1)[R],
+                                          bool (&live)[R])
+{
+#pragma unroll
+  for (int r = 0; r < R; ++r) k0[r] = k1[r] = 0;
+#pragma unroll 1
+  for (int k = 0; k < P.num_keys; ++k) {
+    const KeyCol& c = P.keys[k];
+    const int64_t at = first + c.offset;
+    uint64_t x[R];
+    uint32_t valid[R];
+    auto load = [&](auto* p) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) x[r] = live[r] ? (uint64_t)__ldg(p + at + 32 * r) : 0;
+    };
+    switch (c.width) {
+      case 1: load((const uint8_t*)c.data); break;
+      case 2: load((const uint16_t*)c.data); break;
+      case 4: load((const uint32_t*)c.data); break;
+      default: load((const unsigned long long*)c.data); break;
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) valid[r] = 1u;
+    if (c.mask) {
+      const uint32_t* m = c.mask + (at >> 5);  // rows 32 apart: consecutive words, one bit position
+#pragma unroll
+      for (int r = 0; r < R; ++r) valid[r] = live[r] ? __ldg(m + r) >> (at & 31) : 0u;
+    }
+    fold_key_column<KW, R>(P, c, x, valid, k0, k1, live);
+  }
+}
+
 // 16-byte volatile load (generic address: global or shared)
 __device__ __forceinline__ ulonglong2 vload2(const void* p)
 {

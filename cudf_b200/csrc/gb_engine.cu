@@ -19,6 +19,7 @@
 #include "gb_kernels.cuh"
 #include "gb_partition.cuh"
 #include "gb_record.h"
+#include "gb_stage.h"
 
 namespace gb {
 
@@ -486,15 +487,14 @@ int64_t* pinned_regions()
 // E = alpha_m m^2 / sum 2^-M[j], with linear counting m ln(m/V) while E is
 // below 2.5 m and V registers are still zero.  64-bit hashes need no
 // large-range correction.
-double hll_estimate(const std::vector<uint32_t>& regs)
+double hll_estimate(const uint32_t* regs, int count)
 {
-  const double m = (double)regs.size();
+  const double m = (double)count;
+  int ranks[64] = {};
+  for (int i = 0; i < count; ++i) ++ranks[regs[i] & 63u];
+  const int zeros = ranks[0];
   double z = 0;
-  int zeros = 0;
-  for (uint32_t r : regs) {
-    z += std::ldexp(1.0, -(int)r);
-    zeros += r == 0;
-  }
+  for (int r = 63; r >= 0; --r) z += ranks[r] * std::ldexp(1.0, -r);
   const double alpha = 0.7213 / (1.0 + 1.079 / m);
   double e = alpha * m * m / z;
   if (e <= 2.5 * m && zeros > 0) e = m * std::log(m / zeros);
@@ -630,9 +630,12 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
 
   // ---- group-count estimate from a key sample ----
   int64_t est;
-  std::vector<uint32_t> buckets;
+  const uint32_t* buckets = nullptr;  // rows per hash bucket, in this thread's pinned memory
+  std::vector<uint32_t> even;         // stand-in without a sketch
+  constexpr int kNumBuckets = 1 << kBucketBits;
   bool exact_buckets = false;  // buckets hold exact row counts (full-pass sketch)
   int64_t nsamp = 0;
+  int filled = 0;  // buckets with rows
   if (opt.groups_hint >= 0) {
     est = std::max<int64_t>(1, opt.groups_hint);
   } else if (n <= 65536) {
@@ -660,13 +663,15 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
     ck(cudaMemcpyAsync(hs, hll, ((size_t(1) << kHllBits) + (size_t(1) << kBucketBits)) * 4, cudaMemcpyDeviceToHost,
                        stream), "sketch d2h");
     ck(cudaStreamSynchronize(stream), "sketch sync");
-    std::vector<uint32_t> regs(hs, hs + (size_t(1) << kHllBits));
-    buckets.assign(hs + (size_t(1) << kHllBits), hs + (size_t(1) << kHllBits) + (size_t(1) << kBucketBits));
+    buckets = hs + (size_t(1) << kHllBits);
     S.put(hll);
     exact_buckets = true;
     int64_t valid_rows = 0;
-    for (auto b : buckets) valid_rows += b;
-    est = (int64_t)std::llround(hll_estimate(regs));
+    for (int b = 0; b < kNumBuckets; ++b) {
+      valid_rows += buckets[b];
+      filled += buckets[b] > 0;
+    }
+    est = (int64_t)std::llround(hll_estimate(hs, 1 << kHllBits));
     est = std::min<int64_t>(std::max<int64_t>(est, valid_rows > 0 ? 1 : 0), valid_rows);
     est = std::max<int64_t>(est, 1);
     nsamp = valid_rows;
@@ -674,23 +679,6 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   st.est_groups = est;
   uint32_t rule_fields = 0;
   st.rule = apply_tuning_rules(opt, n, est, P.key_words, &rule_fields);
-  // Many heavy hitters (a long-tailed key distribution, e.g. Zipf): besides
-  // the few partitions well above the average size, most partitions hold keys
-  // with hundreds of rows, whose lanes would queue on one shared address, so
-  // every partition combines the rows of one slot per warp first.  The sign is
-  // in the exact bucket counts: at least 32 buckets above four times the mean
-  // of the non-empty ones (uniform keys have none; one hot key makes one).
-  if (exact_buckets && !((opt.set_mask | rule_fields) & OPT_WAGG)) {
-    int64_t rows_in = 0, nonempty = 0;
-    for (auto b : buckets) {
-      rows_in += b;
-      nonempty += b > 0;
-    }
-    const double mean = nonempty ? (double)rows_in / (double)nonempty : 0.0;
-    int heavy = 0;
-    for (auto b : buckets) heavy += (double)b > 4.0 * mean;
-    if (heavy >= 32) opt.wagg_pct = 0;
-  }
   mark("estimate");
 
   // ---- mode ----
@@ -737,10 +725,18 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   constexpr int kMaxParts = 8192;
   int nparts = 0;
   if (part_ok) {
+    const int64_t sms = dev.sms;
     const int64_t want = std::max<int64_t>(2, (int64_t)std::ceil((double)est / (scap_rec * opt.part_fill)));
-    const int64_t whole = (want + dev.sms - 1) / dev.sms * dev.sms;
     const int64_t tight = (int64_t)std::ceil((double)est / (scap_rec * std::max(opt.part_fill, 0.78)));
-    nparts = (int)(whole <= 2048 ? whole : (int64_t)std::min<uint64_t>(kMaxParts, next_pow2((uint64_t)tight)));
+    // A partition per 32Ki rows, up to four per SM, keeps partitions whole (a
+    // split one's tables all merge into the global table), as long as each
+    // still has 128 groups: with fewer, the rows of a warp queue on few slots
+    // (20M rows, 400 groups over 148 partitions 2.35 ms, over 2 split ones 0.68).
+    const int64_t spread = std::min<int64_t>(4, (n + 32768 * sms - 1) / (32768 * sms)) * sms;
+    const int64_t whole = (std::max(want, std::min(spread, est / 128 / sms * sms)) + sms - 1) / sms * sms;
+    if (want < sms && est < 128 * sms) nparts = (int)std::max(want, est / 128);
+    else if (whole <= 2048) nparts = (int)whole;
+    else nparts = (int)std::min<uint64_t>(kMaxParts, next_pow2((uint64_t)tight));
   }
   const bool part_fits = (double)est <= 0.85 * (double)kMaxParts * sfill2;
   int mode;
@@ -754,23 +750,34 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   // region sizes of the partitioned path: exact rows per partition from the
   // full-pass sketch (else the sample's share with slack)
   std::vector<int64_t> pbase, pend, prows;
+  std::vector<uint8_t> phot;  // partitions that hold a hot key
+  bool long_tail = false;
   if (mode == 2) {
-    if (buckets.empty()) {  // no sketch (hint given or small input): uniform regions
-      buckets.assign((size_t)1 << kBucketBits, 1);
-      nsamp = (int64_t)buckets.size();
-      exact_buckets = false;
+    if (!buckets) {  // no sketch (hint given or small input): uniform regions
+      even.assign(kNumBuckets, 1);
+      buckets = even.data();
+      nsamp = kNumBuckets;
     }
-    constexpr int64_t kBuckets = 1 << kBucketBits;
-    auto first_bucket = [&](int64_t p) { return (p * kBuckets + nparts - 1) / nparts; };  // see part_of
+    auto first_bucket = [&](int64_t p) { return (p * kNumBuckets + nparts - 1) / nparts; };  // see part_of
+    phot.resize(nparts);
+    const double mean = (double)nsamp / std::max(1, filled);
+    for (int b = 0, over = 0; exact_buckets && b < kNumBuckets; ++b)
+      if ((double)buckets[b] > 4 * mean && ++over == 32) long_tail = true;
     pbase.resize(nparts);
     pend.resize(nparts);
     prows.resize(nparts);
     int64_t total = 0, maxload = 0;
-    double samp = 0;
-    for (auto b : buckets) samp += b;
+    const double samp = (double)nsamp;
     for (int p = 0; p < nparts; ++p) {
       double c = 0;
-      for (int64_t b = first_bucket(p); b < first_bucket(p + 1); ++b) c += buckets[b];
+      uint32_t top = 0;
+      for (int64_t b = first_bucket(p); b < first_bucket(p + 1); ++b) {
+        c += buckets[b];
+        top = std::max(top, buckets[b]);
+      }
+      // a key with an eighth of the partition's rows (four lanes of a warp)
+      // shows as a bucket that far above the usual one
+      phot[p] = exact_buckets && (((double)top - mean) * 8 > c || est < 16 * (int64_t)nparts);
       int64_t capp;
       if (exact_buckets) {
         capp = (int64_t)c;
@@ -849,27 +856,33 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
     {
       int64_t nrows = 0;
       for (auto r : prows) nrows += r;
-      // a work item is at most a partition's average share, and small
-      // enough that few partitions still spread over every SM
-      // (a multiple of 64 rows: pass 2 reads rows in pairs from even starts)
-      const int64_t chunk = std::max<int64_t>(
-        32768, std::min<int64_t>(nrows / std::max(1, nparts), nrows / (4 * (int64_t)dev.sms))) & ~(int64_t)63;
-      for (int p = 0; p < nparts; ++p) {
-        const int64_t r = prows[p];
-        if (exact_buckets && r > 2 * chunk) {
-          ++nsplit;
-          for (int64_t b = 0; b < r; b += chunk)
-            items.push_back(PartItem{p, 1, pbase[p] + b, pbase[p] + std::min(r, b + chunk)});
-        }
-      }
-      // whole partitions with well over the average rows hold heavy keys:
-      // they follow the split items into the warp-combining launch
+      // a work item is about a partition's average share, and small enough
+      // that few partitions still spread over every SM (a multiple of 64 rows:
+      // pass 2 reads aligned row pairs)
+      const int64_t share = nrows / std::max(1, nparts);
+      const int64_t chunk =
+        std::max<int64_t>(32768, nparts < dev.sms ? std::min(share, nrows / (4 * (int64_t)dev.sms)) : share) & ~(int64_t)63;
+      // partitions that hold a hot key come first, in the launch that folds
+      // the rows of one slot per warp.  A long-tailed key distribution (32
+      // buckets above four times the usual one: Zipf) has keys of hundreds of
+      // rows everywhere and folds everywhere (100M Zipf pairs: 3.5 ms against
+      // 4.8 with the hottest partitions only).  With wagg_pct given, those
+      // above that share of the average fold.
+      const bool by_share = ((opt.set_mask | rule_fields) & OPT_WAGG) || !exact_buckets;
       const double heavy = opt.wagg_pct / 100.0 * ((double)nrows / std::max(1, nparts));
       for (int pass = 0; pass < 2; ++pass) {
         for (int p = 0; p < nparts; ++p) {
           const int64_t r = prows[p];
-          if (exact_buckets && r > 2 * chunk) continue;
-          if ((pass == 0) == ((double)r > heavy || opt.wagg_pct == 0)) items.push_back(PartItem{p, 0, pbase[p], pend[p]});
+          const bool split = exact_buckets && r > 2 * chunk;
+          const bool folds = by_share ? split || (double)r > heavy || opt.wagg_pct == 0 : long_tail || phot[p];
+          if ((pass == 0) != folds) continue;
+          if (!split) {
+            items.push_back(PartItem{p, 0, pbase[p], pend[p]});
+            continue;
+          }
+          ++nsplit;
+          for (int64_t b = 0; b < r; b += chunk)
+            items.push_back(PartItem{p, 1, pbase[p] + b, pbase[p] + std::min(r, b + chunk)});
         }
         if (pass == 0) nwagg = (int)items.size();
       }
@@ -979,24 +992,31 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
     }
   }
 
-  // shared stage through the row-range kernel: plans whose columns all have
+  // shared stage through k_stage_aggregate: plans whose columns all have
   // closed-form updates and whose groups fit one CTA's ~220 KB table
   bool raw_stage = mode == 1 && part_ok && opt.block >= 512 && !(opt.set_mask & (OPT_SMEM | OPT_FILL)) &&
                    est <= (int64_t)(0.7 * sfill2);
-  std::vector<PartItem> raw_items;
-  PartItem* d_raw_items = nullptr;
-  int64_t* d_raw_spill = nullptr;
-  const uint32_t raw_spill_cap = 1u << 16;
+  bool stage_fold = false;
+  StageArgs stage;
+  std::memset(&stage, 0, sizeof(stage));
   if (!done && raw_stage) {
-    // one row range per CTA for small inputs (each range pays a table reset
-    // and a merge), four per SM for large ones
-    const int64_t per_cta = (n + dev.sms - 1) / dev.sms;
-    const int64_t chunk = per_cta < 4 * 32768 ? per_cta : std::max<int64_t>(32768, (n + 4 * dev.sms - 1) / (4 * dev.sms));
-    for (int64_t b = 0; b < n; b += chunk) raw_items.push_back(PartItem{0, 1, b, std::min(n, b + chunk)});
-    d_raw_items = (PartItem*)S.get(sizeof(PartItem) * raw_items.size());
-    ck(cudaMemcpyAsync(d_raw_items, raw_items.data(), sizeof(PartItem) * raw_items.size(), cudaMemcpyHostToDevice,
-                       stream), "h2d");
-    d_raw_spill = (int64_t*)S.get(sizeof(int64_t) * raw_spill_cap);
+    stage.rows_per_cta = ((n + dev.sms - 1) / dev.sms + 63) & ~(int64_t)63;
+    // copies of the table: as many as fit, while each still sees enough rows
+    // per group to be worth folding back
+    const int64_t slots = std::min<int64_t>(scap_rec, (2 * est + 16 + 3) & ~(int64_t)3);
+    const int64_t fit = scap_rec / slots, worth = stage.rows_per_cta / (16 * est);
+    stage.replicas = (int)std::max<int64_t>(1, std::min<int64_t>(kMaxReplicas, std::min(fit, worth)));
+    stage.slots = (int)(stage.replicas == 1 ? std::min<int64_t>(scap_rec, (4 * est + 64 + 3) & ~(int64_t)3) : slots);
+    stage.sfill = std::max(1, (int)(stage.slots * 0.9));
+    // rows of one slot are folded per warp first where a key may hold a
+    // sixteenth of the rows (two lanes of a warp) and the copies do not
+    // already keep a warp's lanes apart
+    uint32_t top = 0;
+    for (int b = 0; exact_buckets && b < kNumBuckets; ++b) top = std::max(top, buckets[b]);
+    stage_fold = stage.replicas < 32 && (!exact_buckets || (int64_t)top * 16 > n);
+    stage.spill_cap = 1u << 16;
+    stage.spill_rows = (int64_t*)S.get(sizeof(int64_t) * stage.spill_cap);
+    stage.counters = counters;
   }
 
   if (!done) {
@@ -1009,30 +1029,8 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
       int block = std::min(opt.block, 512);
       if (opt.profile) ck(cudaEventRecord(events()[0], stream), "event");
       if (raw_stage) {
-        ck(cudaMemsetAsync(counters + 8, 0, 6 * 4, stream), "memset");  // [8] work, [12..13] spill list
-        PartArgs A;
-        std::memset(&A, 0, sizeof(A));
-        A.counters = counters;
-        A.items = d_raw_items;
-        A.nitems = (int)raw_items.size();
-        A.work = counters + 8;
-        A.spill_rows = d_raw_spill;
-        A.spill_cap = raw_spill_cap;
-        DenseRef D{nullptr, 0, (unsigned long long*)(counters + 10), counters + 6};
-        const size_t sm2 = (size_t)(scap2 + 1) * P.slot_bytes;
-        auto launch_raw = [&](auto kern) {
-          allow_max_smem((const void*)kern);
-          int grid = grid_for((const void*)kern, 1024, sm2, 0);
-          grid = std::min(grid, A.nitems);
-          kern<<<grid, 1024, sm2, stream>>>(P, A, G, D, scap2, sfill2, tmpl);
-        };
-        const bool few = P.num_vals <= 4;
-        if (P.key_words == 1) few ? launch_raw(k_part_aggregate<1, 1, 1024, 4, true, true>)
-                                  : launch_raw(k_part_aggregate<1, 1, 1024, 8, true, true>);
-        else few ? launch_raw(k_part_aggregate<2, 1, 1024, 4, true, true>)
-                 : launch_raw(k_part_aggregate<2, 1, 1024, 8, true, true>);
-        k_part_spill<<<dev.sms * 2, 256, 0, stream>>>(P, G, A);
-        st.kernels += 2;
+        ck(cudaMemsetAsync(counters + 12, 0, 2 * 4, stream), "memset");  // spill list
+        st.kernels += launch_stage(P, stage, G, tmpl, stage_fold, stream);
       } else if (mode == 1) {
         size_t sm = (size_t)scap * P.slot_bytes;
         allow_max_smem((const void*)k_aggregate<true>);

@@ -87,6 +87,22 @@ __device__ __forceinline__ int64_t global_slot(const Plan& P, const TableRef& G,
   return i;
 }
 
+// Merges the counters and accumulators of slot `s` into slot `d` of the same
+// key (either may sit in shared or global memory).
+__device__ __forceinline__ void merge_fields(const Plan& P, uint8_t* d, const uint8_t* s)
+{
+  atomicAdd((unsigned int*)(d + P.rows_off), *(const uint32_t*)(s + P.rows_off));
+#pragma unroll 1
+  for (int v = 0; v < P.num_vals; ++v) {
+    int off = P.vals[v].nulls_off;
+    if (off < 0) continue;
+    uint32_t nn = *(const uint32_t*)(s + off);
+    if (nn) atomicAdd((unsigned int*)(d + off), nn);
+  }
+#pragma unroll 1
+  for (int a = 0; a < P.num_accs; ++a) merge_acc(P, P.accs[a], d, s);
+}
+
 // Merges a shared-memory slot into the global table.
 __device__ __forceinline__ void merge_slot(const Plan& P, const TableRef& G, const uint8_t* s,
                                            unsigned int* s_new)
@@ -99,17 +115,7 @@ __device__ __forceinline__ void merge_slot(const Plan& P, const TableRef& G, con
     atomicOr(G.counters + 1, 1u);
     return;
   }
-  uint8_t* d = G.T + gi * (int64_t)G.stride;
-  atomicAdd((unsigned int*)(d + P.rows_off), *(const uint32_t*)(s + P.rows_off));
-#pragma unroll 1
-  for (int v = 0; v < P.num_vals; ++v) {
-    int off = P.vals[v].nulls_off;
-    if (off < 0) continue;
-    uint32_t nn = *(const uint32_t*)(s + off);
-    if (nn) atomicAdd((unsigned int*)(d + off), nn);
-  }
-#pragma unroll 1
-  for (int a = 0; a < P.num_accs; ++a) merge_acc(P, P.accs[a], d, s);
+  merge_fields(P, G.T + gi * (int64_t)G.stride, s);
 }
 
 // One pass over rows [0, num_rows).  With USE_SMEM each CTA first aggregates
@@ -430,89 +436,94 @@ constexpr int kBucketBits = 14;
 constexpr int kHllBits = 12;
 inline size_t sketch_smem() { return ((size_t(1) << kHllBits) + (size_t(1) << kBucketBits)) * 4; }
 
+// Keys other than one plain 64-bit column are packed four rows per thread; a
+// warp's rows are consecutive, its next step's lines on their way into L2.
+// While the keys of a warp repeat (few groups, or a hot key), rows of one
+// bucket are counted by one lane: 32 lanes adding to the same few counters
+// queue on them.
 static __global__ void __launch_bounds__(512) k_sketch(const __grid_constant__ Plan P, unsigned int* hll,
                                                        unsigned int* buckets)
 {
+  constexpr int NT = 512;
   extern __shared__ unsigned int sk[];
   unsigned int* reg = sk;
   unsigned int* bk = sk + (1 << kHllBits);
-  for (int i = threadIdx.x; i < (1 << kHllBits) + (1 << kBucketBits); i += blockDim.x) sk[i] = 0;
+  for (int i = threadIdx.x; i < (1 << kHllBits) + (1 << kBucketBits); i += NT) sk[i] = 0;
   __syncthreads();
   const int64_t n = P.num_rows;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  auto add = [&](uint64_t h, unsigned rows) {
-    atomicAdd(&bk[h >> (64 - kBucketBits)], rows);
+  auto see = [&](uint64_t h) {  // registers only rise, and soon rarely: read before the atomic
     const uint64_t low = h << 24;
     const unsigned rank = low ? (unsigned)__clzll((long long)low) + 1u : 41u;
-    atomicMax(&reg[(h >> 40) & ((1u << kHllBits) - 1)], rank);
+    unsigned int* r = &reg[(h >> 40) & ((1u << kHllBits) - 1)];
+    if (*(volatile unsigned int*)r < rank) atomicMax(r, rank);
+  };
+  auto add = [&](uint64_t h) {
+    atomicAdd(&bk[h >> (64 - kBucketBits)], 1u);
+    see(h);
   };
   if (P.num_keys == 1 && !P.keys[0].mask && P.keys[0].width == 8 && P.keys[0].cat != CAT_F64) {
     // one plain 64-bit key: four rows per thread in flight
+    const int64_t stride = (int64_t)gridDim.x * NT;
     const unsigned long long* kd = (const unsigned long long*)P.keys[0].data + P.keys[0].offset;
-    int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    int64_t row = blockIdx.x * (int64_t)NT + threadIdx.x;
     for (; row + 3 * stride < n; row += 4 * stride) {
       uint64_t k[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) k[j] = __ldg(kd + row + j * stride);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) add(fmix64(k[j]), 1u);
+      for (int j = 0; j < 4; ++j) add(fmix64(k[j]));
     }
-    for (; row < n; row += stride) add(fmix64(__ldg(kd + row)), 1u);
+    for (; row < n; row += stride) add(fmix64(__ldg(kd + row)));
   } else {
-    // several key columns, nullable or floating-point keys: four rows per
-    // thread, packed column by column so that the four rows' data and mask
-    // loads of a column are in flight together (as pack_key, per row)
     constexpr int SR = 4;
-    for (int64_t row0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; row0 < n; row0 += SR * stride) {
-      uint64_t w0[SR], w1[SR];
-      bool ok[SR];
+    const int lane = threadIdx.x & 31;
+    const int64_t step = (int64_t)gridDim.x * NT * SR;
+    // a lane's line of the warp's step (32 SR rows of one key column)
+    const uint8_t* line = nullptr;
+    int line_w = 0;
+    int left = lane;
+    for (int k = 0; k < P.num_keys; ++k) {
+      const KeyCol& c = P.keys[k];
+      const int lines = (32 * SR * c.width + 127) / 128;
+      if (left >= 0 && left < lines) {
+        line = (const uint8_t*)c.data + c.offset * c.width + left * 128;
+        line_w = c.width;
+      }
+      left -= lines;
+    }
+    bool repeats = false;
+    int since = 0;
+    for (int64_t w0 = (blockIdx.x * (int64_t)NT + (threadIdx.x & ~31)) * SR; w0 < n; w0 += step) {
+      if (line && w0 + step + 32 * SR <= n) asm volatile("prefetch.global.L2 [%0];" ::"l"(line + (w0 + step) * line_w));
+      uint64_t k0[SR], k1[SR];
+      bool live[SR];
+#pragma unroll
+      for (int j = 0; j < SR; ++j) live[j] = w0 + lane + 32 * j < n;
+      pack_rows<2, SR>(P, w0 + lane, k0, k1, live);
+      const bool look = (since++ & 15) == 0;
+      if (look) repeats = false;
 #pragma unroll
       for (int j = 0; j < SR; ++j) {
-        w0[j] = 0;
-        w1[j] = 0;
-        ok[j] = row0 + j * stride < n;
-      }
-#pragma unroll 1
-      for (int k = 0; k < P.num_keys; ++k) {
-        const KeyCol& c = P.keys[k];
-        uint64_t b[SR];
-        uint32_t mw[SR];
-#pragma unroll
-        for (int j = 0; j < SR; ++j) {
-          const int64_t r = row0 + j * stride + c.offset;
-          b[j] = ok[j] ? load_bits(c.data, r, c.width) : 0;
-          mw[j] = (ok[j] && c.mask) ? __ldg(c.mask + (r >> 5)) : 0xFFFFFFFFu;
-        }
-#pragma unroll
-        for (int j = 0; j < SR; ++j) {
-          if (!ok[j]) continue;
-          const int64_t r = row0 + j * stride + c.offset;
-          if (!((mw[j] >> (r & 31)) & 1u)) {
-            if (!P.include_nulls) {
-              ok[j] = false;
-              continue;
-            }
-            const uint64_t nb = 1ull << c.null_shift;
-            if (c.null_word == 0) w0[j] |= nb;
-            else w1[j] |= nb;
-            continue;
+        const uint64_t h = hash_key(k0[j], k1[j], P.key_words);
+        if (repeats || look) {
+          const unsigned b = (unsigned)(h >> (64 - kBucketBits));
+          const unsigned peers = __match_any_sync(0xFFFFFFFFu, live[j] ? b : 0x80000000u);
+          if (look) repeats = repeats || __reduce_max_sync(0xFFFFFFFFu, live[j] ? (unsigned)__popc(peers) : 0u) >= 8;
+          if (live[j]) {
+            if (lane == __ffs(peers) - 1) atomicAdd(&bk[b], __popc(peers));
+            see(h);
           }
-          const uint64_t v = norm_key_bits(c, b[j]) << c.shift;
-          if (c.word == 0) w0[j] |= v;
-          else w1[j] |= v;
+        } else if (live[j]) {
+          add(h);
         }
       }
-#pragma unroll
-      for (int j = 0; j < SR; ++j)
-        if (ok[j]) add(hash_key(w0[j], w1[j], P.key_words), 1u);
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < (1 << kHllBits); i += blockDim.x)
+  for (int i = threadIdx.x; i < (1 << kHllBits); i += NT)
     if (reg[i]) atomicMax(hll + i, reg[i]);
-  for (int i = threadIdx.x; i < (1 << kBucketBits); i += blockDim.x)
+  for (int i = threadIdx.x; i < (1 << kBucketBits); i += NT)
     if (bk[i]) atomicAdd(buckets + i, bk[i]);
 }
-
 
 }  // namespace gb

@@ -8,6 +8,24 @@
 
 namespace gb {
 
+RecCol rec_col(const ValCol& c, int bit, int shift, int adv)
+{
+  const bool nothing = c.sum_off < 0 && c.min_off < 0 && c.max_off < 0 && c.sq_off < 0;
+  const uint32_t kind = nothing               ? RK_NONE
+                        : c.cat == CAT_F64    ? RK_F64
+                        : c.cat == CAT_F32    ? RK_F32
+                        : c.width == 8        ? RK_W64
+                        : c.cat == CAT_SIGNED ? RK_S32
+                                              : RK_Z32;
+  const uint32_t flags = (c.cat == CAT_SIGNED ? RF_SIGNED : 0) | (c.cat == CAT_BOOL ? RF_BOOL : 0) |
+                         (c.sum_op == OP_SUM_I32 ? RF_SUM32 : 0);
+  const uint32_t ext = c.width < 4 ? 32 - 8 * c.width : 0;
+  return RecCol{{(uint32_t)(uint16_t)c.sum_off | (uint32_t)(uint16_t)c.min_off << 16,
+                 (uint32_t)(uint16_t)c.max_off | (uint32_t)(uint16_t)c.sq_off << 16,
+                 (uint32_t)(uint16_t)c.nulls_off | kind << 16 | (uint32_t)shift << 24,
+                 (uint32_t)adv | ext << 8 | flags << 16 | (uint32_t)bit << 24}};
+}
+
 bool record_layout(const Plan& P, RecSpec& S)
 {
   std::memset(&S, 0, sizeof(S));
@@ -54,21 +72,8 @@ bool record_layout(const Plan& P, RecSpec& S)
     const ValCol& c = P.vals[order[j]];
     S.src_col[j] = order[j];
     S.off[j] = at[order[j]];
-    const bool nothing = c.sum_off < 0 && c.min_off < 0 && c.max_off < 0 && c.sq_off < 0;
-    const uint32_t kind = nothing            ? RK_NONE
-                          : c.cat == CAT_F64 ? RK_F64
-                          : c.cat == CAT_F32 ? RK_F32
-                          : c.width == 8     ? RK_W64
-                          : c.cat == CAT_SIGNED ? RK_S32 : RK_Z32;
-    const uint32_t flags = (c.cat == CAT_SIGNED ? RF_SIGNED : 0) | (c.cat == CAT_BOOL ? RF_BOOL : 0) |
-                           (c.sum_op == OP_SUM_I32 ? RF_SUM32 : 0);
-    const uint32_t ext = c.width < 4 ? 32 - 8 * c.width : 0;
-    const uint32_t shift = 8 * (S.off[j] % 8), adv = S.off[j] / 8 - word;
+    S.col[j] = rec_col(c, order[j], 8 * (S.off[j] % 8), S.off[j] / 8 - word);
     word = S.off[j] / 8;
-    S.col[j] = RecCol{{(uint32_t)(uint16_t)c.sum_off | (uint32_t)(uint16_t)c.min_off << 16,
-                       (uint32_t)(uint16_t)c.max_off | (uint32_t)(uint16_t)c.sq_off << 16,
-                       (uint32_t)(uint16_t)c.nulls_off | kind << 16 | shift << 24,
-                       adv | ext << 8 | flags << 16 | (uint32_t)order[j] << 24}};
   }
   for (int v = 0; v < P.num_vals; ++v) {
     if (P.vals[v].mask) {

@@ -135,38 +135,29 @@ __global__ void __launch_bounds__(NT, MINB) k_rec_scatter(const __grid_constant_
       const KeyCol& c = P.keys[kc];
       const int64_t first = t0 + c.offset;
       uint64_t x[RPT];
-      uint32_t valid = 0xFFFFFFFFu;  // bit k: row k
+      uint32_t valid[RPT];
       switch (c.width) {
         case 1: load_rows<uint8_t, NT, RPT>(c.data, first, live, x); break;
         case 2: load_rows<uint16_t, NT, RPT>(c.data, first, live, x); break;
         case 4: load_rows<uint32_t, NT, RPT>(c.data, first, live, x); break;
         default: load_rows<unsigned long long, NT, RPT>(c.data, first, live, x); break;
       }
+#pragma unroll
+      for (int k = 0; k < RPT; ++k) valid[k] = 1u;
       if (c.mask) {
         const int64_t r = first + threadIdx.x;
-        uint32_t w[RPT];
+        const uint32_t* m = c.mask + (r >> 5);  // rows NT apart: NT / 32 words apart, one bit position
 #pragma unroll
-        for (int k = 0; k < RPT; ++k) w[k] = live[k] != 0xFFFFFFFFu ? __ldg(c.mask + ((r + k * NT) >> 5)) : 0u;
-        valid = 0;
-#pragma unroll
-        for (int k = 0; k < RPT; ++k) valid |= ((w[k] >> (r & 31)) & 1u) << k;
+        for (int k = 0; k < RPT; ++k) valid[k] = live[k] != 0xFFFFFFFFu ? __ldg(m + k * (NT / 32)) >> (r & 31) : 0u;
       }
+      bool in[RPT];
 #pragma unroll
-      for (int k = 0; k < RPT; ++k) {
-        if (live[k] == 0xFFFFFFFFu) continue;
-        uint64_t v = norm_key_bits(c, x[k]) << c.shift;
-        int word = c.word;
-        if (!((valid >> k) & 1u)) {
-          if (!P.include_nulls) {
-            live[k] = 0xFFFFFFFFu;
-            continue;
-          }
-          v = 1ull << c.null_shift;
-          word = c.null_word;
-        }
-        if (KW == 1 || word == 0) kw0[k] |= v;
-        else kw1[k] |= v;
-      }
+      for (int k = 0; k < RPT; ++k) in[k] = live[k] != 0xFFFFFFFFu;
+      if constexpr (KW == 2) fold_key_column<2, RPT>(P, c, x, valid, kw0, kw1, in);
+      else fold_key_column<1, RPT>(P, c, x, valid, kw0, kw0, in);
+#pragma unroll
+      for (int k = 0; k < RPT; ++k)
+        if (!in[k]) live[k] = 0xFFFFFFFFu;
     }
   };
   for (int q = threadIdx.x; q < A.nparts; q += NT) hist[q] = 0;
@@ -620,14 +611,87 @@ __device__ __forceinline__ uint32_t rec_slot(const RecTable& t, uint64_t w0, uin
 // letting their updates queue on the slot.
 constexpr int kFoldFrom = 4;
 
+// The columns of R rows per thread into their slots sa (0: no row).  Column j's
+// bits come out of the front word of `rec`, which moves up by the words its
+// descriptor names; validity bits in vb.  One copy of the per-kind update code
+// is looped over the columns (an unrolled copy per column does not fit the
+// instruction cache), so its dispatch is paid once per R rows.  With FOLD, a
+// warp in which a slot occurs kFoldFrom times or more folds the rows of one
+// slot before their updates.  Every lane of a warp calls it.
+template <int R, int RW, bool FOLD>
+__device__ __forceinline__ void apply_columns(const RecSpec& S, int nc, int rows_off, const uint32_t (&sa)[R],
+                                              const unsigned (&vb)[R], uint64_t (&rec)[R][RW])
+{
+  const int lane = threadIdx.x & 31;
+  LaneChain L{0, 0, 0};
+  if constexpr (FOLD) {
+    bool fold = false;  // a slot occurs often enough in the warp to fold its rows first
+    int most[R];
+    unsigned peers[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      peers[r] = __match_any_sync(0xFFFFFFFFu, sa[r] ? sa[r] : (0x80000000u | (unsigned)lane));
+      most[r] = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)__popc(peers[r]));
+      fold = fold || most[r] >= kFoldFrom;
+    }
+    if (fold) {
+      // one row of the thread at a time
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        L = lane_chain(peers[r], most[r]);
+        const bool lead[1] = {sa[r] != 0 && lane == __ffs(peers[r]) - 1};
+        const uint32_t at[1] = {sa[r]};
+        if (lead[0]) sred_add_u32(sa[r] + rows_off, __popc(peers[r]));
+#pragma unroll 1
+        for (int j = 0; j < nc; ++j) {
+          const RecCol c = S.col[j];
+          for (int a = 0; a < c.adv(); ++a) {
+#pragma unroll
+            for (int q = 0; q + 1 < RW; ++q) rec[r][q] = rec[r][q + 1];
+          }
+          const bool valid = (vb[r] >> c.bit()) & 1;
+          if (c.nulls() >= 0) {
+            const unsigned ng = peers[r] & __ballot_sync(0xFFFFFFFFu, sa[r] != 0 && !valid);
+            if (lead[0] && ng) sred_add_u32(sa[r] + c.nulls(), __popc(ng));
+          }
+          const uint64_t x[1] = {rec[r][0] >> c.shift()};
+          const bool ok[1] = {sa[r] != 0 && valid};
+          rec_update<true, 1>(c, at, x, ok, lead, L);
+        }
+      }
+      return;
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (sa[r]) sred_add_u32(sa[r] + rows_off, 1u);
+#pragma unroll 1
+  for (int j = 0; j < nc; ++j) {
+    const RecCol c = S.col[j];
+    for (int a = 0; a < c.adv(); ++a) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+#pragma unroll
+        for (int q = 0; q + 1 < RW; ++q) rec[r][q] = rec[r][q + 1];
+      }
+    }
+    uint64_t x[R];
+    bool ok[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const bool valid = (vb[r] >> c.bit()) & 1;
+      ok[r] = sa[r] != 0 && valid;
+      x[r] = rec[r][0] >> c.shift();
+      if (c.nulls() >= 0 && sa[r] != 0 && !valid) sred_add_u32(sa[r] + c.nulls(), 1u);
+    }
+    rec_update<false, R>(c, sa, x, ok, ok, L);
+  }
+}
+
 // Pass 2.  One CTA owns a work item at a time and aggregates its records in a
 // shared table of `scap` slots (plus the all-ones key's).  Every thread takes
 // R records per step (a warp 32 R consecutive ones), the records two steps
-// ahead being on their way into L2.  The column loop runs one copy of the
-// per-kind update code over the columns (an unrolled copy per column does not
-// fit the instruction cache), so its dispatch is paid once per R rows; a
-// column's bits come out of the front word of the register record, which moves
-// up by a word where the next column begins.
+// ahead being on their way into L2.
 template <int KW, int RW, bool WAGG>
 __global__ void __launch_bounds__(1024, 1) k_rec_aggregate(const __grid_constant__ Plan P,
                                                            const __grid_constant__ RecArgs A,
@@ -699,75 +763,7 @@ __global__ void __launch_bounds__(1024, 1) k_rec_aggregate(const __grid_constant
         }
       }
       __syncwarp();
-      auto advance = [&](int words) {
-        for (int a = 0; a < words; ++a) {
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-#pragma unroll
-            for (int q = 0; q + 1 < RW; ++q) rec[r][q] = rec[r][q + 1];
-          }
-        }
-      };
-      LaneChain L{0, 0, 0};
-      bool fold = false;  // a slot occurs often enough in the warp to fold its rows first
-      int most[R];
-      unsigned peers[R];
-      if (WAGG) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          peers[r] = __match_any_sync(0xFFFFFFFFu, sa[r] ? sa[r] : (0x80000000u | (unsigned)lane));
-          most[r] = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)__popc(peers[r]));
-          fold = fold || most[r] >= kFoldFrom;
-        }
-      }
-      if (WAGG && fold) {
-        // one row of the thread at a time
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          L = lane_chain(peers[r], most[r]);
-          const bool lead[1] = {sa[r] != 0 && lane == __ffs(peers[r]) - 1};
-          const uint32_t at[1] = {sa[r]};
-          if (lead[0]) sred_add_u32(sa[r] + rows_off, __popc(peers[r]));
-          uint64_t word[RW];
-#pragma unroll
-          for (int q = 0; q < RW; ++q) word[q] = rec[r][q];
-#pragma unroll 1
-          for (int j = 0; j < nc; ++j) {
-            const RecCol c = S.col[j];
-            for (int a = 0; a < c.adv(); ++a) {
-#pragma unroll
-              for (int q = 0; q + 1 < RW; ++q) word[q] = word[q + 1];
-            }
-            const bool valid = (vb[r] >> c.bit()) & 1;
-            if (c.nulls() >= 0) {
-              const unsigned ng = peers[r] & __ballot_sync(0xFFFFFFFFu, sa[r] != 0 && !valid);
-              if (lead[0] && ng) sred_add_u32(sa[r] + c.nulls(), __popc(ng));
-            }
-            const uint64_t x[1] = {word[0] >> c.shift()};
-            const bool ok[1] = {sa[r] != 0 && valid};
-            rec_update<true, 1>(c, at, x, ok, lead, L);
-          }
-        }
-        continue;
-      }
-#pragma unroll
-      for (int r = 0; r < R; ++r)
-        if (sa[r]) sred_add_u32(sa[r] + rows_off, 1u);
-#pragma unroll 1
-      for (int j = 0; j < nc; ++j) {
-        const RecCol c = S.col[j];
-        advance(c.adv());
-        uint64_t x[R];
-        bool ok[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const bool valid = (vb[r] >> c.bit()) & 1;
-          ok[r] = sa[r] != 0 && valid;
-          x[r] = rec[r][0] >> c.shift();
-          if (c.nulls() >= 0 && sa[r] != 0 && !valid) sred_add_u32(sa[r] + c.nulls(), 1u);
-        }
-        rec_update<false, R>(c, sa, x, ok, ok, L);
-      }
+      apply_columns<R, RW, WAGG>(S, nc, rows_off, sa, vb, rec);
     }
     __syncthreads();
     p2_flush<NT, ScanT>(P, G, D, slots, scap, s_spill != 0 || item.merge, scan_tmp, &s_base, &s_new);

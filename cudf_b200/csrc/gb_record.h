@@ -70,6 +70,9 @@ struct RecArgs {
   unsigned int* work;            // pass 2 claim counter
 };
 
+// Descriptor of a value column: validity bit, bit position in its word, words
+// since the previous column's.
+RecCol rec_col(const ValCol& c, int bit, int shift, int adv);
 // Lays the record out; false when the plan has no record form (more than
 // kMaxRecCols value columns).
 bool record_layout(const Plan& P, RecSpec& S);
