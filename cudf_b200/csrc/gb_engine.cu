@@ -182,7 +182,7 @@ static uint64_t next_pow2(uint64_t x)
 // ---------------------------------------------------------------------------
 // planning
 void build_plan(const std::vector<Column>& keys, int null_policy, const std::vector<Request>& reqs,
-                Plan& P, std::vector<int>& out_types)
+                Plan& P, std::vector<int>& out_types, bool wide_f32)
 {
   std::memset(&P, 0, sizeof(P));
   if (keys.empty()) throw Error(ERR_LOGIC, "groupby needs at least one key column");
@@ -263,6 +263,7 @@ void build_plan(const std::vector<Column>& keys, int null_policy, const std::vec
   P.num_vals = (int)vk.size();
 
   // which accumulator ops each column needs
+  const uint8_t sq_f32 = wide_f32 ? OP_SQ_F64 : OP_SQ_F32;
   std::vector<std::vector<uint8_t>> ops(vk.size());
   std::vector<bool> need_nulls(vk.size(), false), need_m2(vk.size(), false);
   auto add = [&](int v, uint8_t op) {
@@ -278,7 +279,7 @@ void build_plan(const std::vector<Column>& keys, int null_policy, const std::vec
       int k = reqs[r].aggs[j].kind;
       if (c.mask && k != K_COUNT_ALL) need_nulls[v] = true;
       auto sum_op = [&]() -> uint8_t {
-        if (cat == CAT_F32) return OP_SUM_F32;
+        if (cat == CAT_F32) return wide_f32 ? OP_SUM_F64 : OP_SUM_F32;
         if (cat == CAT_F64) return OP_SUM_F64;
         if (is_dur(t) && w == 4) return OP_SUM_I32;
         return OP_SUM_I64;
@@ -288,7 +289,7 @@ void build_plan(const std::vector<Column>& keys, int null_policy, const std::vec
         case K_VARIANCE: case K_STD: add(v, sum_op()); need_m2[v] = true; break;
         case K_MIN: add(v, w == 8 ? OP_MIN_U64 : OP_MIN_U32); break;
         case K_MAX: add(v, w == 8 ? OP_MAX_U64 : OP_MAX_U32); break;
-        case K_SUM_OF_SQUARES: add(v, cat == CAT_F32 ? OP_SQ_F32 : cat == CAT_F64 ? OP_SQ_F64 : OP_SQ_I64); break;
+        case K_SUM_OF_SQUARES: add(v, cat == CAT_F32 ? sq_f32 : cat == CAT_F64 ? OP_SQ_F64 : OP_SQ_I64); break;
         case K_PRODUCT: add(v, cat == CAT_F32 ? OP_PROD_F32 : cat == CAT_F64 ? OP_PROD_F64 : OP_PROD_I64); break;
         case K_ARGMIN: add(v, w == 8 ? OP_ARGMIN_R64 : OP_ARGMIN_P32); P.has_arg = 1; break;
         case K_ARGMAX: add(v, w == 8 ? OP_ARGMAX_R64 : OP_ARGMAX_P32); P.has_arg = 1; break;
@@ -320,6 +321,7 @@ void build_plan(const std::vector<Column>& keys, int null_policy, const std::vec
     c.nulls_off = -1;
     c.sum_off = -1;
     c.m2_off = -1;
+    c.wide = wide_f32 && c.cat == CAT_F32;
     if (need_nulls[v]) { c.nulls_off = (int16_t)off; off += 4; }
   }
   // accumulators grouped per column, 4-byte ones first within the slot
@@ -406,7 +408,7 @@ void build_plan(const std::vector<Column>& keys, int null_policy, const std::vec
         case K_MIN: o.nullable = has_nulls; o.acc_off = acc_for(v, w == 8 ? OP_MIN_U64 : OP_MIN_U32); break;
         case K_MAX: o.nullable = has_nulls; o.acc_off = acc_for(v, w == 8 ? OP_MAX_U64 : OP_MAX_U32); break;
         case K_SUM_OF_SQUARES: o.nullable = has_nulls;
-          o.acc_off = acc_for(v, c.cat == CAT_F32 ? OP_SQ_F32 : c.cat == CAT_F64 ? OP_SQ_F64 : OP_SQ_I64); break;
+          o.acc_off = acc_for(v, c.cat == CAT_F32 ? sq_f32 : c.cat == CAT_F64 ? OP_SQ_F64 : OP_SQ_I64); break;
         case K_PRODUCT: o.nullable = has_nulls;
           o.acc_off = acc_for(v, c.cat == CAT_F32 ? OP_PROD_F32 : c.cat == CAT_F64 ? OP_PROD_F64 : OP_PROD_I64); break;
         case K_ARGMIN: o.nullable = has_nulls; o.acc_off = acc_for(v, w == 8 ? OP_ARGMIN_R64 : OP_ARGMIN_P32); break;
@@ -590,7 +592,7 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   Options opt = opt_in;  // tuning rules may adjust it once the group estimate is known
   Plan P;
   std::vector<int> out_types;
-  build_plan(keys, null_policy, reqs, P, out_types);
+  build_plan(keys, null_policy, reqs, P, out_types, true);
   Stats st;
   Result R;
   R.alloc = alloc;

@@ -123,8 +123,11 @@ struct Stats {
 
 // Builds the plan (validates like cudf::groupby::aggregate,
 // cpp/src/groupby/groupby.cu:202-219, and cpp/src/groupby/groupby.cu:174-190).
+// wide_f32: sums and sums of squares of FLOAT32 columns are held in 64 bits, so
+// that their error does not grow with the rows one table slot takes; the
+// results are rounded to FLOAT32 once.
 void build_plan(const std::vector<Column>& keys, int null_policy, const std::vector<Request>& reqs,
-                Plan& P, std::vector<int>& out_types);
+                Plan& P, std::vector<int>& out_types, bool wide_f32 = false);
 
 // The groupby: keys table + requests -> unique keys and one column per
 // requested aggregation, in request order.

@@ -16,7 +16,7 @@
 
 namespace gb {
 
-constexpr int kMaxSlotBytes = 1024;
+constexpr int kMaxSlotBytes = 1536;
 // Longest probe run of a global table.  At load <= 0.5 linear probing needs a
 // few probes; a run this long means the table is (nearly) full, which is
 // reported as overflow (the host regrows the table) instead of scanning it.
@@ -237,7 +237,7 @@ static __global__ void __launch_bounds__(256) k_var_pass(const __grid_constant__
       double x = (c.cat == CAT_F32 || c.cat == CAT_F64) ? e.d : (c.cat == CAT_UNSIGNED ? (double)e.bits : (double)e.i);
       double sum;
       switch (c.cat) {
-        case CAT_F32: sum = *(const float*)(slot + c.sum_off); break;
+        case CAT_F32: sum = c.wide ? *(const double*)(slot + c.sum_off) : (double)*(const float*)(slot + c.sum_off); break;
         case CAT_F64: sum = *(const double*)(slot + c.sum_off); break;
         default: sum = (double)*(const int64_t*)(slot + c.sum_off); break;
       }
@@ -312,6 +312,7 @@ __device__ __forceinline__ uint64_t finalize(const Plan& P, const OutSpec& o, co
     case K_COUNT_VALID: valid = true; return (uint64_t)cnt;
     case K_COUNT_ALL: valid = true; return rows;
     case K_SUM: case K_SUM_OF_SQUARES: case K_PRODUCT:
+      if (c.wide && o.kind != K_PRODUCT) return __float_as_uint((float)*(const double*)a);
       return o.out_width == 8 ? *(const uint64_t*)a : *(const uint32_t*)a;
     case K_MIN: case K_MAX: {
       bool is_min = o.kind == K_MIN;
@@ -334,7 +335,7 @@ __device__ __forceinline__ uint64_t finalize(const Plan& P, const OutSpec& o, co
         return (uint64_t)(s / cnt);
       }
       double s;
-      if (c.cat == CAT_F32) s = *(const float*)a;
+      if (c.cat == CAT_F32) s = c.wide ? *(const double*)a : (double)*(const float*)a;
       else if (c.cat == CAT_F64) s = *(const double*)a;
       else s = (double)*(const int64_t*)a;
       return (uint64_t)__double_as_longlong(s / (double)cnt);

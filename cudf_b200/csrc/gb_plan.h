@@ -92,6 +92,7 @@ struct ValCol {
   int16_t sq_off;
   uint8_t sum_op;         // OP_SUM_* or 0
   uint8_t basic;          // 1 when every accumulator is a SUM, MIN, MAX or sum of squares
+  uint8_t wide;           // FLOAT32 sums and sums of squares accumulate in f64 (OP_SUM_F64, OP_SQ_F64)
 };
 
 struct Acc {

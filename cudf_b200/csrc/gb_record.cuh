@@ -430,7 +430,8 @@ __device__ __forceinline__ void rec_update(const RecCol& c, const uint32_t (&sa)
     }
     case RK_F32: {
       auto f = [&](int r) { return __uint_as_float((uint32_t)x[r]); };
-      if (so >= 0) sum(so, f, [](uint32_t a, float v) { sred_add_f32(a, v); });
+      auto d = [&](int r) { return (double)f(r); };
+      if (so >= 0) sum(so, d, [](uint32_t a, double v) { sred_add_f64(a, v); });
       if (mo >= 0 || xo >= 0) {
         uint32_t lo[R], hi[R];
 #pragma unroll
@@ -440,7 +441,7 @@ __device__ __forceinline__ void rec_update(const RecCol& c, const uint32_t (&sa)
         }
         min_max32(lo, hi);
       }
-      if (qo >= 0) sum(qo, [&](int r) { return f(r) * f(r); }, [](uint32_t a, float v) { sred_add_f32(a, v); });
+      if (qo >= 0) sum(qo, [&](int r) { return d(r) * d(r); }, [](uint32_t a, double v) { sred_add_f64(a, v); });
       break;
     }
     case RK_W64: {

@@ -88,3 +88,30 @@ def test_table_fill_and_partition_counts(groups):
                       [(cb.Column.from_numpy(v, rng.random(n) > 0.1), wide), (cb.Column.from_numpy(f), wide)],
                       tuning={"force_mode": 2, "part_fill_pct": 85})
     assert gb.stats()["mode"] == 2
+
+
+@pytest.mark.parametrize("mode,n,groups", [(1, 400_000, 3), (1, 2_000_000, 900), (2, 2_000_000, 1), (2, 3_000_000, 4_000),
+                                           (0, 400_000, 5)])
+def test_float32_sums_round_once(mode, n, groups):
+    """FLOAT32 sums, means and sums of squares accumulate in 64 bits: however
+    many rows a group has, SUM is the float nearest to the exact sum up to the
+    64-bit additions' own error (n * 2^-52 of sum|x|, far below half a float
+    step), so at most one float step away."""
+    import cudf_b200 as cb
+    from cudf_b200 import aggregation as agg
+    rng = np.random.default_rng(groups)
+    key = rng.integers(0, groups, n).astype(np.int64)
+    x = rng.lognormal(size=n).astype(np.float32)
+    gb = cb.GroupBy(cb.Table([cb.Column.from_numpy(key)]))
+    gb.set_tuning(force_mode=mode)
+    uk, res = gb.aggregate([cb.GroupByRequest(cb.Column.from_numpy(x), [agg.sum(), agg.mean(), agg.sum_of_squares()])])
+    got = uk[0].to_numpy()[0]
+    x64 = x.astype(np.float64)
+    total = np.bincount(key, x64, groups)[got]
+    count = np.bincount(key, minlength=groups)[got]
+    squares = np.bincount(key, x64 * x64, groups)[got]
+    for values, exact in ((res[0][0], total), (res[0][2], squares)):
+        v = values.to_numpy()[0]
+        assert v.dtype == np.float32
+        assert np.all(np.abs(v.astype(np.float64) - exact) <= np.spacing(exact.astype(np.float32)))
+    assert np.allclose(res[0][1].to_numpy()[0], total / count, rtol=n * 2.0**-52, atol=0)
