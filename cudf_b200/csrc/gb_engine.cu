@@ -145,9 +145,14 @@ void Result::release()
   auto fr = [&](void* p, size_t n) {
     if (p && alloc.deallocate) alloc.deallocate(alloc.ctx, p, n, (void*)stream);
   };
-  for (auto& c : keys) { fr(c.data, c.data_bytes); fr(c.mask, c.mask_bytes); }
-  for (auto& r : results)
-    for (auto& c : r) { fr(c.data, c.data_bytes); fr(c.mask, c.mask_bytes); }
+  if (block) {
+    fr(block, block_bytes);
+    block = nullptr;
+  } else {
+    for (auto& c : keys) { fr(c.data, c.data_bytes); fr(c.mask, c.mask_bytes); }
+    for (auto& r : results)
+      for (auto& c : r) { fr(c.data, c.data_bytes); fr(c.mask, c.mask_bytes); }
+  }
   keys.clear();
   results.clear();
 }
@@ -622,8 +627,10 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
 
   Scratch S(alloc, stream);
   mark("begin");
-  unsigned int* counters = (unsigned int*)S.get(4096);
-  ck(cudaMemsetAsync(counters, 0, 4096, stream), "memset counters");
+  const bool sketch = opt.groups_hint < 0 && n > 65536;
+  const size_t sketch_bytes = sketch ? sketch_smem() : 0;
+  unsigned int* counters = (unsigned int*)S.get(4096 + sketch_bytes);
+  ck(cudaMemsetAsync(counters, 0, 4096 + sketch_bytes, stream), "memset counters");
   mark("counters");
   uint32_t* host = pinned();
   DevInfo dev = dev_info();
@@ -640,15 +647,13 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   int filled = 0;  // buckets with rows
   if (opt.groups_hint >= 0) {
     est = std::max<int64_t>(1, opt.groups_hint);
-  } else if (n <= 65536) {
+  } else if (!sketch) {
     est = n;
   } else {
     // full pass over the keys: exact rows per hash bucket (partition region
     // sizes) and a HyperLogLog estimate of the number of distinct keys
-    unsigned int* hll = (unsigned int*)S.get((sizeof(unsigned int) << kHllBits) + (sizeof(unsigned int) << kBucketBits));
+    unsigned int* hll = counters + 1024;
     unsigned int* bk = hll + (1 << kHllBits);
-    ck(cudaMemsetAsync(hll, 0, (sizeof(unsigned int) << kHllBits) + (sizeof(unsigned int) << kBucketBits), stream),
-       "memset sketch");
     {
       const size_t sm = sketch_smem();
       allow_max_smem((const void*)k_sketch);
@@ -666,7 +671,6 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
                        stream), "sketch d2h");
     ck(cudaStreamSynchronize(stream), "sketch sync");
     buckets = hs + (size_t(1) << kHllBits);
-    S.put(hll);
     exact_buckets = true;
     int64_t valid_rows = 0;
     for (int b = 0; b < kNumBuckets; ++b) {
@@ -711,7 +715,7 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   const int scap_rec = std::max(0, std::min(220 * 1024, dev.smem_optin - 8192) / (P.slot_bytes + 4) - 1) & ~3;  // with tags
   const int scap2 = std::max(0, std::min(220 * 1024, dev.smem_optin - 8192) / P.slot_bytes - 1);
   const int sfill2 = std::max(1, (int)(scap2 * 0.8));
-  bool part_ok = !P.has_arg && !P.need_second_pass && P.num_vals <= 8 && scap2 >= 256;
+  bool part_ok = !P.has_arg && P.num_vals <= 8 && scap2 >= 256;
   for (int v = 0; v < P.num_vals; ++v) part_ok = part_ok && P.vals[v].basic;
   for (int a = 0; a < P.num_accs; ++a) {
     uint8_t op = P.accs[a].op;
@@ -811,6 +815,7 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   int64_t dense_n = 0;
   int64_t dense_cap = 0;
   bool done = false;
+  bool clean = true;  // counters still as cleared at the start
   // one read-back for the whole call (see Options::sync_checks)
   const bool deferred = !opt.sync_checks;
   bool prof_part = false, prof_agg = false;
@@ -879,7 +884,8 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
           const bool folds = by_share ? split || (double)r > heavy || opt.wagg_pct == 0 : long_tail || phot[p];
           if ((pass == 0) != folds) continue;
           if (!split) {
-            items.push_back(PartItem{p, 0, pbase[p], pend[p]});
+            // VARIANCE/STD: the second pass looks every group up in the global table
+            items.push_back(PartItem{p, P.need_second_pass, pbase[p], pend[p]});
             continue;
           }
           ++nsplit;
@@ -890,7 +896,7 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
       }
       // CTAs claim items in order: largest first within each launch, so the
       // launch does not end waiting on one long item taken last
-      auto rows_of = [&](const PartItem& it) { return it.merge ? it.end - it.begin : prows[it.part]; };
+      auto rows_of = [&](const PartItem& it) { return std::min(it.end - it.begin, prows[it.part]); };
       auto larger = [&](const PartItem& x, const PartItem& y) { return rows_of(x) > rows_of(y); };
       std::stable_sort(items.begin(), items.begin() + nwagg, larger);
       std::stable_sort(items.begin() + nwagg, items.end(), larger);
@@ -906,7 +912,8 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
     // groups expected to miss their partition's shared table, plus those of
     // split partitions, go to the global spill table
     const double expect_spill = std::max(0.0, (double)est - 0.85 * (double)nparts * sfill2);
-    uint64_t spill_cap = next_pow2((uint64_t)std::max<double>(65536.0, 2.0 * expect_spill + 2.0 * (double)nsplit * scap2));
+    uint64_t spill_cap = next_pow2((uint64_t)std::max<double>(65536.0, 2.0 * expect_spill + 2.0 * (double)nsplit * scap2 +
+                                                                              (P.need_second_pass ? 2.0 * est : 0.0)));
     // spill list: room for the rows of the groups expected to spill
     uint32_t spill_list = (uint32_t)std::min<uint64_t>(
       1ull << 31, next_pow2((uint64_t)std::max<double>(262144.0, 4.0 * expect_spill)));
@@ -918,9 +925,9 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
       A.spill_rows = (int64_t*)S.get((size_t)spill_list * sizeof(int64_t));
       A.spill_cap = spill_list;
       k_init_slots<<<dev.sms * 4, 256, 0, stream>>>(T, (int64_t)spill_cap + 1, P.slot_bytes, tmpl);
-      ck(cudaMemsetAsync(counters, 0, 16, stream), "memset");
+      if (attempt > 0) ck(cudaMemsetAsync(counters, 0, 16, stream), "memset");
       // [6] dense overflow, [8..9] work, [10..11] dense count, [12] spill list length, [13] list overflow
-      ck(cudaMemsetAsync(counters + 6, 0, 8 * 4, stream), "memset");
+      if (attempt > 0) ck(cudaMemsetAsync(counters + 6, 0, 8 * 4, stream), "memset");
       G = TableRef{T, spill_cap - 1, P.slot_bytes, P.key_words, counters};
       DenseRef D{dense, dcap, (unsigned long long*)(counters + 10), counters + 6};
       // items of split (heavy) partitions first, with rows of one slot
@@ -942,8 +949,8 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
       // sample sized the partitions well): one grid-stride launch that reads
       // the list length on the device
       launch_rec_spill(P, A, rec, G, dev.sms * 2, stream);
-      k_finish_count<<<1, 1, 0, stream>>>(P, G);
-      st.kernels += 3;
+      if (!deferred) k_finish_count<<<1, 1, 0, stream>>>(P, G);  // deferred: the compaction counts it
+      st.kernels += deferred ? 2 : 3;
       ck(cudaGetLastError(), "partition aggregate launch");
       if (deferred) {
         // counts and flags stay on the device until the compaction is done
@@ -984,6 +991,7 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
       ++st.retries;
     }
     if (!done) {
+      clean = false;
       mode = 0;
       st.mode = 0;
       ++st.retries;
@@ -1026,12 +1034,12 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
       size_t tbytes = (size_t)(cap + 1) * P.slot_bytes;
       T = (uint8_t*)S.get(tbytes);
       k_init_slots<<<dev.sms * 8, 256, 0, stream>>>(T, (int64_t)cap + 1, P.slot_bytes, tmpl);
-      ck(cudaMemsetAsync(counters, 0, 16, stream), "memset counters");
+      if (attempt > 0 || !clean) ck(cudaMemsetAsync(counters, 0, 16 * 4, stream), "memset counters");
       G = TableRef{T, cap - 1, P.slot_bytes, P.key_words, counters};
       int block = std::min(opt.block, 512);
       if (opt.profile) ck(cudaEventRecord(events()[0], stream), "event");
       if (raw_stage) {
-        ck(cudaMemsetAsync(counters + 12, 0, 2 * 4, stream), "memset");  // spill list
+        if (attempt > 0) ck(cudaMemsetAsync(counters + 12, 0, 2 * 4, stream), "memset");  // spill list
         st.kernels += launch_stage(P, stage, G, tmpl, stage_fold, stream);
       } else if (mode == 1) {
         size_t sm = (size_t)scap * P.slot_bytes;
@@ -1045,8 +1053,8 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
         k_aggregate<false><<<grid, block, 0, stream>>>(P, G, 1, 0, tmpl);
       }
       if (opt.profile) ck(cudaEventRecord(events()[1], stream), "event");
-      k_finish_count<<<1, 1, 0, stream>>>(P, G);
-      st.kernels += 3;
+      if (!deferred) k_finish_count<<<1, 1, 0, stream>>>(P, G);
+      st.kernels += deferred ? 2 : 3;
       ck(cudaGetLastError(), "aggregate launch");
       if (deferred) {
         prof_agg = opt.profile;
@@ -1091,29 +1099,67 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   try {
     OutPtrs O;
     std::memset(&O, 0, sizeof(O));
-    for (int k = 0; k < P.num_keys; ++k) {
-      R.keys.push_back(make_out(alloc, stream, keys[k].type_id, out_rows, keys[k].mask != nullptr));
-      O.key_data[k] = R.keys.back().data;
-      O.key_mask[k] = R.keys.back().mask;
-    }
+    // every column in one allocation: the data first, then all masks together
+    // (one clear for them, and for a small call most of its time was the
+    // allocations and clears of its columns)
     {
+      auto column = [&](int type_id) {
+        OutColumn c;
+        c.type_id = type_id;
+        c.size = out_rows;
+        return c;
+      };
+      for (int k = 0; k < P.num_keys; ++k) R.keys.push_back(column(keys[k].type_id));
       int j = 0;
       for (auto& r : reqs) {
         std::vector<OutColumn> cols;
-        for (size_t a = 0; a < r.aggs.size(); ++a, ++j) {
-          cols.push_back(make_out(alloc, stream, out_types[j], out_rows, P.outs[j].nullable));
-          O.out_data[j] = cols.back().data;
-          O.out_mask[j] = cols.back().mask;
-        }
+        for (size_t q = 0; q < r.aggs.size(); ++q) cols.push_back(column(out_types[j++]));
         R.results.push_back(cols);
       }
+      const size_t rows = (size_t)std::max<int64_t>(out_rows, 1);
+      const size_t mask_bytes = (rows + 511) / 512 * 64;  // as cudf pads them
+      size_t at = 0;
+      auto take = [&](size_t bytes) {
+        const size_t o = at;
+        at += (bytes + 255) & ~(size_t)255;
+        return o;
+      };
+      std::vector<size_t> data_at, mask_at;
+      auto each = [&](auto f) {
+        for (int k = 0; k < P.num_keys; ++k) f(R.keys[k], keys[k].mask != nullptr);
+        int o = 0;
+        for (auto& cols : R.results)
+          for (auto& c : cols) f(c, P.outs[o++].nullable != 0);
+      };
+      each([&](OutColumn& c, bool) { data_at.push_back(take(rows * type_width(c.type_id))); });
+      const size_t masks = at;
+      each([&](OutColumn&, bool nullable) { mask_at.push_back(nullable ? take(mask_bytes) : 0); });
+      R.block_bytes = std::max<size_t>(at, 16);
+      R.block = alloc.allocate(alloc.ctx, R.block_bytes, (void*)stream);
+      if (!R.block) throw Error(ERR_ALLOC, "device allocation of the output columns failed");
+      if (at > masks) ck(cudaMemsetAsync((uint8_t*)R.block + masks, 0, at - masks, stream), "memset masks");
+      size_t i = 0;
+      each([&](OutColumn& c, bool nullable) {
+        c.data = (uint8_t*)R.block + data_at[i];
+        c.mask = nullable ? (uint32_t*)((uint8_t*)R.block + mask_at[i]) : nullptr;
+        ++i;
+      });
+      for (int k = 0; k < P.num_keys; ++k) {
+        O.key_data[k] = R.keys[k].data;
+        O.key_mask[k] = R.keys[k].mask;
+      }
+      j = 0;
+      for (auto& cols : R.results)
+        for (auto& c : cols) {
+          O.out_data[j] = c.data;
+          O.out_mask[j++] = c.mask;
+        }
     }
     // position and null counters of the compaction, apart from the
-    // aggregation's counts and flags in counters[0, 16)
+    // aggregation's counts and flags in counters[0, 16); cleared with them
     unsigned int* ccount = counters + 256;
     uint32_t* chost = host + 256;
     O.counters = ccount;
-    ck(cudaMemsetAsync(ccount, 0, 512, stream), "memset");
     if (opt.profile) ck(cudaEventRecord(events()[2], stream), "event");
     const int64_t limit = deferred ? out_rows : G_n;
     if (deferred && dense) {
@@ -1134,9 +1180,10 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
     }
     if (opt.profile) ck(cudaEventRecord(events()[3], stream), "event");
     ck(cudaGetLastError(), "compact launch");
-    if (deferred) ck(cudaMemcpyAsync(host, counters, 64, cudaMemcpyDeviceToHost, stream), "counts d2h");
-    ck(cudaMemcpyAsync(chost, ccount, 4 * (4 + P.num_keys + P.num_outs), cudaMemcpyDeviceToHost, stream),
-       "null counts d2h");
+    // deferred: the counts and flags come with the compaction's counters
+    const int ncc = 4 + P.num_keys + P.num_outs;
+    if (deferred) ck(cudaMemcpyAsync(host, counters, 4 * (256 + ncc), cudaMemcpyDeviceToHost, stream), "counts d2h");
+    else ck(cudaMemcpyAsync(chost, ccount, 4 * ncc, cudaMemcpyDeviceToHost, stream), "null counts d2h");
     ck(cudaStreamSynchronize(stream), "compact sync");
     mark("compaction (synced)");
     if (deferred) {
@@ -1152,9 +1199,9 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
       }
       const int64_t dn = mode == 2 ? (int64_t)(host[10] | ((uint64_t)host[11] << 32)) : 0;
       G_n = (int64_t)chost[2];
-      if (G_n != (int64_t)host[0] + dn)
+      if (G_n != (int64_t)host[0] + dn + chost[3])
         throw Error(ERR_CUDA, "internal error: compaction wrote " + std::to_string(G_n) + " groups of " +
-                                  std::to_string((int64_t)host[0] + dn));
+                                  std::to_string((int64_t)host[0] + dn + chost[3]));
       R.num_groups = G_n;
       for (auto& c : R.keys) c.size = G_n;
       for (auto& cols : R.results)

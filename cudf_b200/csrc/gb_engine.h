@@ -63,6 +63,9 @@ struct Result {
   std::vector<std::vector<OutColumn>> results;
   Allocator alloc{};
   cudaStream_t stream = nullptr;
+  // one allocation holding every column (null: each column owns its buffers)
+  void* block = nullptr;
+  size_t block_bytes = 0;
   void release();  // frees every buffer through alloc
 };
 

@@ -259,7 +259,7 @@ struct OutPtrs {
   uint32_t* key_mask[kMaxKeyCols];
   void* out_data[kMaxOutputs];
   uint32_t* out_mask[kMaxOutputs];
-  unsigned int* counters;  // [2] output position, [4 + j] null count of output column j
+  unsigned int* counters;  // [2] output position, [3] 1 when the all-ones key is a group, [4 + j] null count of output column j
 };
 
 __device__ __forceinline__ void store_width(void* base, int64_t i, int width, uint64_t bits)
@@ -368,6 +368,7 @@ __device__ __forceinline__ void compact_block(const Plan& P, const uint8_t* T, i
   int64_t i = base + threadIdx.x;
   const uint8_t* slot = T + i * (int64_t)stride;
   bool occ = i < nslots && (dense || slot_occupied(P, slot, i == nslots - 1));
+  if (occ && !dense && i == nslots - 1) atomicAdd(O.counters + 3, 1u);
   int local, total;
   Scan(tmp).ExclusiveSum(occ ? 1 : 0, local, total);
   if (threadIdx.x == 0) *s_base = total ? atomicAdd(O.counters + 2, (unsigned)total) : 0;
