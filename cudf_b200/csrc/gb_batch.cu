@@ -24,7 +24,7 @@
 
 #include "../../include/cudf_b200.h"
 #include "gb_batch.h"
-#include "gb_stage.cuh"
+#include "gb_kernels.cuh"
 
 namespace gb {
 
@@ -240,140 +240,6 @@ static __global__ void __launch_bounds__(NT) k_batch_aggregate(const __grid_cons
   }
 }
 
-// A row straight into its instance's global table (out of line: the hot loop
-// keeps its registers).
-static __device__ __noinline__ void batch_global_row(const Plan& P, uint8_t* T, uint64_t cap_mask, unsigned int* counters,
-                                                     uint64_t w0, uint64_t w1, int64_t row, unsigned int* s_new)
-{
-  const TableRef G{T, cap_mask, P.slot_bytes, P.key_words, counters};
-  const int64_t gi = global_slot(P, G, w0, w1, hash_key(w0, w1, P.key_words), s_new);
-  if (gi < 0) atomicOr(counters + 1, 1u);
-  else update_slot(P, T + gi * (int64_t)P.slot_bytes, row);
-}
-
-// A shared slot into the instance's global table, or into slot `d` of another copy.
-static __device__ __noinline__ void batch_merge(const Plan& P, uint8_t* T, uint64_t cap_mask, unsigned int* counters,
-                                                const uint8_t* s, uint8_t* d, unsigned int* s_new)
-{
-  if (d) merge_fields(P, d, s);
-  else merge_slot(P, TableRef{T, cap_mask, P.slot_bytes, P.key_words, counters}, s, s_new);
-}
-
-// The same for schemas whose columns all have closed-form updates (sums, MIN,
-// MAX, sums of squares; at most eight columns): tagged shared tables and the
-// per-kind column updates of the partitioned path, R rows per thread.  An
-// instance with few groups keeps several copies of its table in the tile, as
-// in k_stage_aggregate.  `budget` = shared slots a tile has.
-template <int KW, int MAXV>
-static __global__ void __launch_bounds__(1024, 1) k_batch_columns(const __grid_constant__ Plan P,
-                                                                  const __grid_constant__ RecSpec S,
-                                                                  const BatchInst* insts, const BatchTile* tiles,
-                                                                  int64_t ntiles, int budget,
-                                                                  const __grid_constant__ SlotTemplate tmpl)
-{
-  constexpr int NT = 1024;
-  constexpr int R = MAXV <= 4 ? 2 : 1;
-  extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ __align__(16) Plan sp;
-  __shared__ unsigned int s_used[kMaxReplicas];
-  __shared__ unsigned int s_new;
-  for (int i = threadIdx.x; i < (int)(sizeof(Plan) / 4); i += NT) ((uint32_t*)&sp)[i] = ((const uint32_t*)&P)[i];
-  const int stride = P.slot_bytes;
-  const int nw = stride / 8;
-  const int nc = S.ncols;
-  const int lane = threadIdx.x & 31;
-  const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
-  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    __syncthreads();
-    const BatchTile tl = tiles[t];
-    const BatchInst& I = insts[tl.inst];
-    const int scap = I.scap;
-    // an instance whose table overflowed is re-run with a larger table: skip
-    const int64_t end = *(volatile unsigned int*)(I.counters + 1) ? tl.begin : tl.end;
-    int copies = 0;
-    if (scap > 0)
-      copies = (int)max((int64_t)1, min((int64_t)min(kMaxReplicas, budget / scap), (tl.end - tl.begin) / (8 * (int64_t)scap)));
-    const int total = copies * scap;
-    uint8_t* const slots = smem + (size_t)total * 4;
-    if (threadIdx.x == 0) {
-      patch_plan(sp, I);
-      s_new = 0;
-    }
-    for (int i = threadIdx.x; i < copies; i += NT) s_used[i] = 0;
-    for (int i = threadIdx.x; i < total / 4; i += NT) ((uint4*)smem)[i] = make_uint4(0, 0, 0, 0);
-    for (int w = 0; w < nw; ++w) {
-      const unsigned long long x = tmpl.w[w];
-      for (int s = threadIdx.x; s < total; s += NT) *(unsigned long long*)(slots + ((size_t)s * nw + w) * 8) = x;
-    }
-    __syncthreads();
-    auto table_of = [&](int copy) {
-      return RecTable{sbase + 4u * (uint32_t)(copy * scap), sbase + 4u * (uint32_t)total + (uint32_t)(copy * scap * stride),
-                      (uint32_t)scap / 4, stride, I.sfill, (uint32_t)__cvta_generic_to_shared(s_used + copy)};
-    };
-    const RecTable table = table_of(copies > 0 ? threadIdx.x % copies : 0);
-    int since_check = 0;
-    for (int64_t w0 = tl.begin + (threadIdx.x >> 5) * (32 * R); w0 < end; w0 += R * NT) {
-      if (++since_check == 32) {
-        since_check = 0;
-        if (__any_sync(0xFFFFFFFFu, *(volatile unsigned int*)(I.counters + 1) != 0)) break;
-      }
-      const int64_t row = w0 + lane;
-      uint64_t k0[R], k1[R], x[R][MAXV];
-      bool live[R];
-      unsigned vb[R];
-      uint32_t sa[R];
-#pragma unroll
-      for (int r = 0; r < R; ++r) live[r] = row + 32 * r < end;
-      pack_rows<KW, R>(sp, row, k0, k1, live);
-      if (total > 0) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) vb[r] = 0xFFu;
-#pragma unroll
-        for (int v = 0; v < MAXV; ++v) {
-          if (v >= nc) break;
-          const ValCol& c = sp.vals[v];
-          const int64_t at = row + c.offset;
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            x[r][v] = live[r] ? load_bits(c.data, at + 32 * r, c.width) : 0;
-            if (c.mask && live[r] && !((__ldg(c.mask + ((at + 32 * r) >> 5)) >> (at & 31)) & 1u)) vb[r] &= ~(1u << v);
-          }
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        sa[r] = 0;
-        if (!live[r]) continue;
-        const uint64_t h = hash_key(k0[r], k1[r], KW);
-        if (total > 0 && !(KW == 1 && k0[r] == kEmpty)) sa[r] = rec_slot<KW>(table, k0[r], k1[r], h);
-        if (sa[r] == 0) {  // no shared table, or no room in it
-          batch_global_row(sp, I.table, I.cap_mask, I.counters, k0[r], k1[r], row + 32 * r, &s_new);
-        }
-      }
-      __syncwarp();
-      if (total > 0) apply_columns<R, MAXV, true>(S, nc, P.rows_off, sa, vb, x, copies < 8);
-    }
-    __syncthreads();
-    if (copies > 1) {
-      const RecTable first = table_of(0);
-      for (int i = scap + threadIdx.x; i < total; i += NT) {
-        const uint8_t* s = slots + (size_t)i * stride;
-        if (!slot_occupied(sp, s, false)) continue;
-        const uint64_t w0 = ((const uint64_t*)s)[0], w1 = KW == 2 ? ((const uint64_t*)s)[1] : 0;
-        const uint32_t d = rec_slot<KW>(first, w0, w1, hash_key(w0, w1, KW));
-        batch_merge(sp, I.table, I.cap_mask, I.counters, s, d ? (uint8_t*)__cvta_shared_to_generic(d) : nullptr, &s_new);
-      }
-      __syncthreads();
-    }
-    for (int i = threadIdx.x; i < scap; i += NT) {
-      const uint8_t* s = slots + (size_t)i * stride;
-      if (slot_occupied(sp, s, false)) batch_merge(sp, I.table, I.cap_mask, I.counters, s, nullptr, &s_new);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0 && s_new) atomicAdd(I.counters, s_new);
-  }
-}
-
 static __global__ void k_batch_finish(const __grid_constant__ Plan P, const BatchInst* insts, int ninst)
 {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -479,9 +345,6 @@ struct Batch::Impl {
   unsigned int* h_counters = nullptr;  // pinned copy of the per-instance counters
   size_t counter_words = 128;
   SlotTemplate tmpl;
-  bool columns = false;  // k_batch_columns takes the schema
-  RecSpec rec;
-  int slot_budget = 0;   // shared slots of a tile
   int smem_bytes = 0;
   int grid_agg = 0, grid_compact = 0;
   int block = 512;
@@ -592,22 +455,6 @@ struct Batch::Impl {
     k_batch_aggregate<NT><<<grid_agg, NT, smem_bytes, s>>>(P, (const BatchInst*)d_insts.p, (const BatchTile*)d_tiles.p,
                                                            (int64_t)tiles.size(), (unsigned int*)d_work.p, tmpl);
   }
-  const void* columns_kernel() const
-  {
-    const bool few = P.num_vals <= 4;
-    if (P.key_words == 1) return few ? (const void*)k_batch_columns<1, 4> : (const void*)k_batch_columns<1, 8>;
-    return few ? (const void*)k_batch_columns<2, 4> : (const void*)k_batch_columns<2, 8>;
-  }
-  void launch_columns(cudaStream_t s)
-  {
-    auto go = [&](auto kern) {
-      kern<<<grid_agg, 1024, smem_bytes, s>>>(P, rec, (const BatchInst*)d_insts.p, (const BatchTile*)d_tiles.p,
-                                              (int64_t)tiles.size(), slot_budget, tmpl);
-    };
-    const bool few = P.num_vals <= 4;
-    if (P.key_words == 1) few ? go(k_batch_columns<1, 4>) : go(k_batch_columns<1, 8>);
-    else few ? go(k_batch_columns<2, 4>) : go(k_batch_columns<2, 8>);
-  }
   static const void* agg_kernel(int block)
   {
     switch (block) {
@@ -622,8 +469,7 @@ struct Batch::Impl {
     ck(cudaMemsetAsync(d_counters.p, 0, (size_t)ninst * counter_words * 4, s), "memset counters");
     ck(cudaMemsetAsync(d_work.p, 0, 16, s), "memset work");
     k_batch_init<<<sms * 8, 256, 0, s>>>((uint8_t*)d_tables.p, total_slots, P.slot_bytes, tmpl);
-    if (columns) launch_columns(s);
-    else switch (block) {
+    switch (block) {
       case 256: launch_agg<256>(s); break;
       case 1024: launch_agg<1024>(s); break;
       default: launch_agg<512>(s); break;
@@ -746,16 +592,13 @@ void Batch::prepare(const std::vector<std::vector<Column>>& keys, int null_polic
   }
   // distinct data pointers per request so build_plan keeps one value column per request
   for (size_t r = 0; r < r0.size(); ++r) r0[r].values.data = (const void*)(uintptr_t)(0x1000 + 64 * r);
-  build_plan(k0, null_policy, r0, B.P, B.out_types, true);
+  build_plan(k0, null_policy, r0, B.P, B.out_types);
   if (B.P.need_second_pass) throw Error(ERR_UNSUPPORTED, "VARIANCE/STD are not supported in batched mode");
   B.ninst = ninst;
   B.nout = B.P.num_outs;
   B.A = A;
   B.stream = stream;
   slot_template(B.P, B.tmpl);
-  B.columns = !B.P.has_arg && B.P.num_vals <= kMaxRecCols;
-  for (int v = 0; v < B.P.num_vals; ++v) B.columns = B.columns && B.P.vals[v].basic;
-  if (B.columns) stage_layout(B.P, B.rec);
 
   // instance descriptors (column pointers; tables filled in below)
   B.insts.assign(ninst, BatchInst{});
@@ -808,7 +651,7 @@ void Batch::prepare(const std::vector<std::vector<Column>>& keys, int null_polic
   const int stride = B.P.slot_bytes;
   int scap_max = 1;
   {
-    int budget = std::min(bo.smem_bytes >= 0 ? bo.smem_bytes : launch.smem_bytes, optin - 16384 - (int)sizeof(Plan));
+    int budget = std::min(bo.smem_bytes >= 0 ? bo.smem_bytes : launch.smem_bytes, optin - 8192 - (int)sizeof(Plan));
     while ((int64_t)scap_max * 2 * stride <= budget) scap_max *= 2;
     if (scap_max * stride > budget) scap_max = 0;
   }
@@ -875,12 +718,13 @@ void Batch::prepare(const std::vector<std::vector<Column>>& keys, int null_polic
        "h2d");
   if (!B.h_counters) ck(cudaMallocHost((void**)&B.h_counters, (size_t)ninst * B.counter_words * 4), "cudaMallocHost");
   // launch shapes
-  B.slot_budget = scap_max;
-  B.smem_bytes = scap_max * (B.columns ? stride + 4 : stride);  // tags
+  B.smem_bytes = scap_max * stride;
   B.block = launch.block;
   B.stats.block = launch.block;
   B.stats.tile_rows = launch.tile_rows;
-  allow_max_smem(B.columns ? B.columns_kernel() : Impl::agg_kernel(B.block));
+  allow_max_smem(Impl::agg_kernel(B.block));
+  int bps = 0;
+  ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, Impl::agg_kernel(B.block), B.block, B.smem_bytes), "occ");
   B.grid_agg = (int)std::min<int64_t>(std::max<int64_t>(1, (int64_t)B.tiles.size()), 1 << 30);
   B.grid_compact = sms * 8;
   B.stats.instances = ninst;

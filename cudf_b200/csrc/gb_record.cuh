@@ -618,15 +618,14 @@ constexpr int kFoldFrom = 4;
 // is looped over the columns (an unrolled copy per column does not fit the
 // instruction cache), so its dispatch is paid once per R rows.  With FOLD, a
 // warp in which a slot occurs kFoldFrom times or more folds the rows of one
-// slot before their updates (look = false, the same for a warp: it does not
-// look for that).  Every lane of a warp calls it.
+// slot before their updates.  Every lane of a warp calls it.
 template <int R, int RW, bool FOLD>
 __device__ __forceinline__ void apply_columns(const RecSpec& S, int nc, int rows_off, const uint32_t (&sa)[R],
-                                              const unsigned (&vb)[R], uint64_t (&rec)[R][RW], bool look = true)
+                                              const unsigned (&vb)[R], uint64_t (&rec)[R][RW])
 {
   const int lane = threadIdx.x & 31;
   LaneChain L{0, 0, 0};
-  if (FOLD && look) {
+  if constexpr (FOLD) {
     bool fold = false;  // a slot occurs often enough in the warp to fold its rows first
     int most[R];
     unsigned peers[R];
