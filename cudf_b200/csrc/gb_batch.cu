@@ -268,7 +268,7 @@ static __global__ void __launch_bounds__(256) k_batch_compact(const __grid_const
     const BatchInst& I = insts[ch.inst];
     const int64_t nslots = (int64_t)I.cap_mask + 2;
     const int64_t limit = *(volatile const unsigned int*)I.counters;
-    compact_block(P, I.table, nslots, P.slot_bytes, limit, 0, outs[ch.inst], ch.base, &tmp, &s_base);
+    compact_block(P, I.table, nslots, P.slot_bytes, limit, outs[ch.inst], ch.base, &tmp, &s_base);
   }
 }
 

@@ -471,8 +471,9 @@ cudaEvent_t* events()
   return t_ev;
 }
 // Per-thread pinned host words: [0, 1024) counters read back by the host,
-// [1024, 1024 + 2^kHllBits + 2^kBucketBits) the key sketch.
-constexpr size_t kPinnedWords = 1024 + (size_t(1) << kHllBits) + (size_t(1) << kBucketBits);
+// [1024, 1040) the sample flag, then 2^kHllBits + 2^kBucketBits words of the key
+// sketch.
+constexpr size_t kPinnedWords = 1024 + 16 + (size_t(1) << kHllBits) + (size_t(1) << kBucketBits);
 uint32_t* pinned()
 {
   if (!t_pinned) ck(cudaMallocHost((void**)&t_pinned, kPinnedWords * 4), "cudaMallocHost");
@@ -625,10 +626,16 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
     return R;
   }
 
+  constexpr int kNumBuckets = 1 << kBucketBits;
   Scratch S(alloc, stream);
   mark("begin");
   const bool sketch = opt.groups_hint < 0 && n > 65536;
-  const size_t sketch_bytes = sketch ? sketch_smem() : 0;
+  // From 8M rows on a sample of 512Ki rows is looked at first: with few groups
+  // it is the sketch (60M rows of six groups: 0.31 ms for all of them), else it
+  // costs about 12 us ahead of the pass over all rows (0.1 to 0.7 ms).
+  constexpr int64_t kSampleFrom = 8 << 20, kSampleChunks = 4096;
+  const bool sample = sketch && !opt.full_sketch && n >= kSampleFrom;
+  const size_t sketch_bytes = (sketch ? sketch_smem() : 0) * (sample ? 2 : 1) + (sketch ? 64 : 0);
   unsigned int* counters = (unsigned int*)S.get(4096 + sketch_bytes);
   ck(cudaMemsetAsync(counters, 0, 4096 + sketch_bytes, stream), "memset counters");
   mark("counters");
@@ -641,10 +648,10 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   int64_t est;
   const uint32_t* buckets = nullptr;  // rows per hash bucket, in this thread's pinned memory
   std::vector<uint32_t> even;         // stand-in without a sketch
-  constexpr int kNumBuckets = 1 << kBucketBits;
   bool exact_buckets = false;  // buckets hold exact row counts (full-pass sketch)
   int64_t nsamp = 0;
   int filled = 0;  // buckets with rows
+  bool sampled = false;  // the sketch is a sample's
   if (opt.groups_hint >= 0) {
     est = std::max<int64_t>(1, opt.groups_hint);
   } else if (!sketch) {
@@ -652,26 +659,33 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   } else {
     // full pass over the keys: exact rows per hash bucket (partition region
     // sizes) and a HyperLogLog estimate of the number of distinct keys
-    unsigned int* hll = counters + 1024;
+    unsigned int* few = counters + 1024;  // flag, then registers and buckets, then the sample's
+    unsigned int* hll = few + 16;
     unsigned int* bk = hll + (1 << kHllBits);
     {
       const size_t sm = sketch_smem();
       allow_max_smem((const void*)k_sketch);
       // at least 16Ki rows per CTA: each CTA clears and merges 80 KB of
       // shared counters, which dominates on small inputs
-      int grid = grid_for((const void*)k_sketch, 512, sm, 0);
-      grid = (int)std::min<int64_t>(grid, (n + 16383) / 16384);
-      k_sketch<<<grid, 512, sm, stream>>>(P, hll, bk);
+      const int full = grid_for((const void*)k_sketch, 512, sm, 0);
+      int grid = (int)std::min<int64_t>(full, (n + 16383) / 16384);
+      if (sample) {
+        unsigned int* shll = bk + kNumBuckets;
+        k_sketch<<<std::min(full, 128), 512, sm, stream>>>(P, shll, shll + (1 << kHllBits), kSampleChunks, nullptr);
+        k_sketch_few<<<1, 1024, 0, stream>>>(shll, hll, few);
+        st.kernels += 2;
+      }
+      k_sketch<<<grid, 512, sm, stream>>>(P, hll, bk, 0, sample ? few : nullptr);
     }
     st.kernels += 1;
     ck(cudaGetLastError(), "sketch launch");
     mark("sketch launched");
-    uint32_t* hs = host + 1024;  // registers then buckets, adjacent on the device too
-    ck(cudaMemcpyAsync(hs, hll, ((size_t(1) << kHllBits) + (size_t(1) << kBucketBits)) * 4, cudaMemcpyDeviceToHost,
-                       stream), "sketch d2h");
+    uint32_t* hs = host + 1024 + 16;  // registers then buckets, adjacent on the device too
+    ck(cudaMemcpyAsync(hs - 16, few, 64 + sketch_smem(), cudaMemcpyDeviceToHost, stream), "sketch d2h");
     ck(cudaStreamSynchronize(stream), "sketch sync");
     buckets = hs + (size_t(1) << kHllBits);
-    exact_buckets = true;
+    sampled = sample && hs[-16] != 0;
+    exact_buckets = !sampled;
     int64_t valid_rows = 0;
     for (int b = 0; b < kNumBuckets; ++b) {
       valid_rows += buckets[b];
@@ -753,6 +767,12 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   if (mode == 1 && scap < 16) mode = 0;
   if (mode == 2 && !part_ok) mode = 0;
 
+  if (sampled && mode != 1) {  // only the shared stage does without every row's count
+    Options o2 = opt_in;
+    o2.full_sketch = 1;
+    return aggregate(keys, null_policy, reqs, stream, alloc, o2, stats);
+  }
+
   // region sizes of the partitioned path: exact rows per partition from the
   // full-pass sketch (else the sample's share with slack)
   std::vector<int64_t> pbase, pend, prows;
@@ -811,14 +831,83 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
 
   uint8_t* T = nullptr;
   TableRef G{};
-  uint8_t* dense = nullptr;
-  int64_t dense_n = 0;
-  int64_t dense_cap = 0;
   bool done = false;
   bool clean = true;  // counters still as cleared at the start
   // one read-back for the whole call (see Options::sync_checks)
   const bool deferred = !opt.sync_checks;
   bool prof_part = false, prof_agg = false;
+
+  // position and null counters of the result rows, apart from the
+  // aggregation's counts and flags in counters[0, 16); cleared with them
+  unsigned int* ccount = counters + 256;
+  uint32_t* chost = host + 256;
+  OutPtrs O;
+  std::memset(&O, 0, sizeof(O));
+  O.counters = ccount;
+  struct Undo {  // the outputs go back when the call does not return them
+    Result& r;
+    bool keep = false;
+    ~Undo() { if (!keep) r.release(); }
+  } undo{R};
+  auto make_outputs = [&](int64_t out_rows) {
+    // every column in one allocation: the data first, then all masks together
+    // (one clear for them, and for a small call most of its time was the
+    // allocations and clears of its columns)
+    {
+      auto column = [&](int type_id) {
+        OutColumn c;
+        c.type_id = type_id;
+        c.size = out_rows;
+        return c;
+      };
+      for (int k = 0; k < P.num_keys; ++k) R.keys.push_back(column(keys[k].type_id));
+      int j = 0;
+      for (auto& r : reqs) {
+        std::vector<OutColumn> cols;
+        for (size_t q = 0; q < r.aggs.size(); ++q) cols.push_back(column(out_types[j++]));
+        R.results.push_back(cols);
+      }
+      const size_t rows = (size_t)std::max<int64_t>(out_rows, 1);
+      const size_t mask_bytes = (rows + 511) / 512 * 64;  // as cudf pads them
+      size_t at = 0;
+      auto take = [&](size_t bytes) {
+        const size_t o = at;
+        at += (bytes + 255) & ~(size_t)255;
+        return o;
+      };
+      std::vector<size_t> data_at, mask_at;
+      auto each = [&](auto f) {
+        for (int k = 0; k < P.num_keys; ++k) f(R.keys[k], keys[k].mask != nullptr);
+        int o = 0;
+        for (auto& cols : R.results)
+          for (auto& c : cols) f(c, P.outs[o++].nullable != 0);
+      };
+      each([&](OutColumn& c, bool) { data_at.push_back(take(rows * type_width(c.type_id))); });
+      const size_t masks = at;
+      each([&](OutColumn&, bool nullable) { mask_at.push_back(nullable ? take(mask_bytes) : 0); });
+      R.block_bytes = std::max<size_t>(at, 16);
+      R.block = alloc.allocate(alloc.ctx, R.block_bytes, (void*)stream);
+      if (!R.block) throw Error(ERR_ALLOC, "device allocation of the output columns failed");
+      if (at > masks) ck(cudaMemsetAsync((uint8_t*)R.block + masks, 0, at - masks, stream), "memset masks");
+      size_t i = 0;
+      each([&](OutColumn& c, bool nullable) {
+        c.data = (uint8_t*)R.block + data_at[i];
+        c.mask = nullable ? (uint32_t*)((uint8_t*)R.block + mask_at[i]) : nullptr;
+        ++i;
+      });
+      for (int k = 0; k < P.num_keys; ++k) {
+        O.key_data[k] = R.keys[k].data;
+        O.key_mask[k] = R.keys[k].mask;
+      }
+      j = 0;
+      for (auto& cols : R.results)
+        for (auto& c : cols) {
+          O.out_data[j] = c.data;
+          O.out_mask[j++] = c.mask;
+        }
+    }
+  };
+  int64_t out_rows = -1;
 
   if (mode == 2) {
     // ---- pass 1: scatter rows into hash partitions ----
@@ -884,8 +973,9 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
           const bool folds = by_share ? split || (double)r > heavy || opt.wagg_pct == 0 : long_tail || phot[p];
           if ((pass == 0) != folds) continue;
           if (!split) {
-            // VARIANCE/STD: the second pass looks every group up in the global table
-            items.push_back(PartItem{p, P.need_second_pass, pbase[p], pend[p]});
+            // VARIANCE/STD: the second pass looks every group up in the global
+            // table; with checks after each stage the groups are counted there
+            items.push_back(PartItem{p, P.need_second_pass || !deferred, pbase[p], pend[p]});
             continue;
           }
           ++nsplit;
@@ -913,23 +1003,27 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
     // split partitions, go to the global spill table
     const double expect_spill = std::max(0.0, (double)est - 0.85 * (double)nparts * sfill2);
     uint64_t spill_cap = next_pow2((uint64_t)std::max<double>(65536.0, 2.0 * expect_spill + 2.0 * (double)nsplit * scap2 +
-                                                                              (P.need_second_pass ? 2.0 * est : 0.0)));
+                                                                              (P.need_second_pass || !deferred ? 2.0 * est : 0.0)));
     // spill list: room for the rows of the groups expected to spill
     uint32_t spill_list = (uint32_t)std::min<uint64_t>(
       1ull << 31, next_pow2((uint64_t)std::max<double>(262144.0, 4.0 * expect_spill)));
     int64_t dcap = (int64_t)(est * 1.5) + (int64_t)nparts * 256 + 4096;
-    dense_cap = dcap;
     for (int attempt = 0;; ++attempt) {
       T = (uint8_t*)S.get((size_t)(spill_cap + 1) * P.slot_bytes);
-      dense = (uint8_t*)S.get((size_t)dcap * P.slot_bytes);
       A.spill_rows = (int64_t*)S.get((size_t)spill_list * sizeof(int64_t));
       A.spill_cap = spill_list;
       k_init_slots<<<dev.sms * 4, 256, 0, stream>>>(T, (int64_t)spill_cap + 1, P.slot_bytes, tmpl);
       if (attempt > 0) ck(cudaMemsetAsync(counters, 0, 16, stream), "memset");
-      // [6] dense overflow, [8..9] work, [10..11] dense count, [12] spill list length, [13] list overflow
+      // [8..9] work, [10..11] groups written by pass 2, [12] spill list length, [13] list overflow
       if (attempt > 0) ck(cudaMemsetAsync(counters + 6, 0, 8 * 4, stream), "memset");
       G = TableRef{T, spill_cap - 1, P.slot_bytes, P.key_words, counters};
-      DenseRef D{dense, dcap, (unsigned long long*)(counters + 10), counters + 6};
+      // result rows for every group pass 2 writes and every slot of T; with
+      // checks after each stage, pass 2 merges everything into T instead
+      if (deferred) {
+        out_rows = dcap + (int64_t)spill_cap + 1;
+        make_outputs(out_rows);
+      }
+      const EmitRef D{out_rows, (unsigned long long*)(counters + 10)};
       // items of split (heavy) partitions first, with rows of one slot
       // combined per warp before their shared update; then the rest
       auto launch2 = [&](int first, int count, unsigned int* work, bool wagg) {
@@ -938,7 +1032,7 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
         Ai.items = d_items + first;
         Ai.nitems = count;
         Ai.work = work;
-        (P.key_words == 1 ? launch_rec_aggregate1 : launch_rec_aggregate2)(P, Ai, rec, G, D, scap_p, sfill_p, tmpl, wagg,
+        (P.key_words == 1 ? launch_rec_aggregate1 : launch_rec_aggregate2)(P, Ai, rec, G, D, O, scap_p, sfill_p, tmpl, wagg,
                                                                            stream);
         ++st.kernels;
       };
@@ -956,7 +1050,6 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
         // counts and flags stay on the device until the compaction is done
         mark("partition passes launched");
         done = true;
-        dense_n = -1;
         cap = spill_cap;
         prof_part = opt.profile;
         break;
@@ -972,21 +1065,18 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
       }
       mark("partition passes (synced)");
       if (host[5]) break;  // a region overflowed: fall back to the global table
-      if (host[1] == 0 && host[6] == 0 && host[13] == 0) {
+      if (host[1] == 0 && host[13] == 0) {
         done = true;
-        dense_n = (int64_t)(host[10] | ((uint64_t)host[11] << 32));
         cap = spill_cap;
         break;
       }
       if (attempt >= 6) throw Error(ERR_CUDA, "hash table overflow");
       if (host[1]) spill_cap *= 8;
-      if (host[6]) dcap *= 2;
       if (host[13]) {
         spill_list = (uint32_t)std::min<uint64_t>((uint64_t)spill_list * 8, 1ull << 31);
         spill_cap = std::max<uint64_t>(spill_cap, next_pow2((uint64_t)host[12] * 2));
       }
       S.put(T);
-      S.put(dense);
       S.put(A.spill_rows);
       ++st.retries;
     }
@@ -996,9 +1086,7 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
       st.mode = 0;
       ++st.retries;
       S.put(T);
-      S.put(dense);
       S.put(A.spill_rows);
-      dense = nullptr;
     }
   }
 
@@ -1022,8 +1110,8 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
     // sixteenth of the rows (two lanes of a warp) and the copies do not
     // already keep a warp's lanes apart
     uint32_t top = 0;
-    for (int b = 0; exact_buckets && b < kNumBuckets; ++b) top = std::max(top, buckets[b]);
-    stage_fold = stage.replicas < 32 && (!exact_buckets || (int64_t)top * 16 > n);
+    for (int b = 0; buckets && b < kNumBuckets; ++b) top = std::max(top, buckets[b]);
+    stage_fold = stage.replicas < 32 && (!buckets || (int64_t)top * 16 > nsamp);
     stage.spill_cap = 1u << 16;
     stage.spill_rows = (int64_t*)S.get(sizeof(int64_t) * stage.spill_cap);
     stage.counters = counters;
@@ -1084,8 +1172,8 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   mark("aggregate done");
   mark("outputs");
   // deferred: outputs are sized for every slot that could hold a group
-  int64_t G_n = deferred ? -1 : (int64_t)host[0] + dense_n;
-  const int64_t out_rows = deferred ? (dense ? dense_cap : 0) + (int64_t)cap + 1 : G_n;
+  int64_t G_n = deferred ? -1 : (int64_t)host[0];
+  if (out_rows < 0) out_rows = deferred ? (int64_t)cap + 1 : G_n;
   R.num_groups = G_n;
 
   if (P.need_second_pass) {
@@ -1096,86 +1184,14 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   }
 
   // ---- outputs ----
-  try {
-    OutPtrs O;
-    std::memset(&O, 0, sizeof(O));
-    // every column in one allocation: the data first, then all masks together
-    // (one clear for them, and for a small call most of its time was the
-    // allocations and clears of its columns)
-    {
-      auto column = [&](int type_id) {
-        OutColumn c;
-        c.type_id = type_id;
-        c.size = out_rows;
-        return c;
-      };
-      for (int k = 0; k < P.num_keys; ++k) R.keys.push_back(column(keys[k].type_id));
-      int j = 0;
-      for (auto& r : reqs) {
-        std::vector<OutColumn> cols;
-        for (size_t q = 0; q < r.aggs.size(); ++q) cols.push_back(column(out_types[j++]));
-        R.results.push_back(cols);
-      }
-      const size_t rows = (size_t)std::max<int64_t>(out_rows, 1);
-      const size_t mask_bytes = (rows + 511) / 512 * 64;  // as cudf pads them
-      size_t at = 0;
-      auto take = [&](size_t bytes) {
-        const size_t o = at;
-        at += (bytes + 255) & ~(size_t)255;
-        return o;
-      };
-      std::vector<size_t> data_at, mask_at;
-      auto each = [&](auto f) {
-        for (int k = 0; k < P.num_keys; ++k) f(R.keys[k], keys[k].mask != nullptr);
-        int o = 0;
-        for (auto& cols : R.results)
-          for (auto& c : cols) f(c, P.outs[o++].nullable != 0);
-      };
-      each([&](OutColumn& c, bool) { data_at.push_back(take(rows * type_width(c.type_id))); });
-      const size_t masks = at;
-      each([&](OutColumn&, bool nullable) { mask_at.push_back(nullable ? take(mask_bytes) : 0); });
-      R.block_bytes = std::max<size_t>(at, 16);
-      R.block = alloc.allocate(alloc.ctx, R.block_bytes, (void*)stream);
-      if (!R.block) throw Error(ERR_ALLOC, "device allocation of the output columns failed");
-      if (at > masks) ck(cudaMemsetAsync((uint8_t*)R.block + masks, 0, at - masks, stream), "memset masks");
-      size_t i = 0;
-      each([&](OutColumn& c, bool nullable) {
-        c.data = (uint8_t*)R.block + data_at[i];
-        c.mask = nullable ? (uint32_t*)((uint8_t*)R.block + mask_at[i]) : nullptr;
-        ++i;
-      });
-      for (int k = 0; k < P.num_keys; ++k) {
-        O.key_data[k] = R.keys[k].data;
-        O.key_mask[k] = R.keys[k].mask;
-      }
-      j = 0;
-      for (auto& cols : R.results)
-        for (auto& c : cols) {
-          O.out_data[j] = c.data;
-          O.out_mask[j++] = c.mask;
-        }
-    }
-    // position and null counters of the compaction, apart from the
-    // aggregation's counts and flags in counters[0, 16); cleared with them
-    unsigned int* ccount = counters + 256;
-    uint32_t* chost = host + 256;
-    O.counters = ccount;
+  {
+    if (!R.block) make_outputs(out_rows);
     if (opt.profile) ck(cudaEventRecord(events()[2], stream), "event");
     const int64_t limit = deferred ? out_rows : G_n;
-    if (deferred && dense) {
-      int grid = (int)std::min<int64_t>((dense_cap + 255) / 256, (int64_t)dev.sms * 8);
-      k_compact<<<grid, 256, 0, stream>>>(P, dense, dense_cap, P.slot_bytes, limit, 1, O,
-                                          (const unsigned long long*)(counters + 10));
-      ++st.kernels;
-    } else if (dense_n > 0) {
-      int grid = (int)std::min<int64_t>((dense_n + 255) / 256, (int64_t)dev.sms * 8);
-      k_compact<<<grid, 256, 0, stream>>>(P, dense, dense_n, P.slot_bytes, limit, 1, O);
-      ++st.kernels;
-    }
-    if (deferred || G_n > dense_n) {
+    if (deferred || G_n > 0) {
       int64_t nslots = (int64_t)cap + 1;
       int grid = (int)std::min<int64_t>((nslots + 255) / 256, (int64_t)dev.sms * 8);
-      k_compact<<<grid, 256, 0, stream>>>(P, T, nslots, P.slot_bytes, limit, 0, O);
+      k_compact<<<grid, 256, 0, stream>>>(P, T, nslots, P.slot_bytes, limit, O);
       ++st.kernels;
     }
     if (opt.profile) ck(cudaEventRecord(events()[3], stream), "event");
@@ -1187,14 +1203,15 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
     ck(cudaStreamSynchronize(stream), "compact sync");
     mark("compaction (synced)");
     if (deferred) {
-      // an overflow anywhere (a table, a region, the dense slots, a spill
+      // an overflow anywhere (a table, a region, the result rows, a spill
       // list): redo the call with checks after every stage
-      const bool again = host[1] || chost[1] || (mode == 2 && (host[5] || host[6] || host[13])) ||
+      const bool again = host[1] || chost[1] || (mode == 2 && (host[5] || host[13])) ||
                          (raw_stage && host[13]);
       if (again) {
         R.release();
         Options o2 = opt_in;
         o2.sync_checks = 1;
+        o2.full_sketch = 1;
         return aggregate(keys, null_policy, reqs, stream, alloc, o2, stats);
       }
       const int64_t dn = mode == 2 ? (int64_t)(host[10] | ((uint64_t)host[11] << 32)) : 0;
@@ -1227,11 +1244,9 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
     int j = 0;
     for (auto& cols : R.results)
       for (auto& c : cols) c.null_count = chost[4 + P.num_keys + j++];
-  } catch (...) {
-    R.release();
-    throw;
   }
   if (stats) *stats = st;
+  undo.keep = true;
   return R;
 }
 
@@ -1324,7 +1339,7 @@ int64_t aggregate_into_scratch(const std::vector<Column>& keys, int null_policy,
     if (G_n > 0) {
       int64_t nslots = (int64_t)cap + 1;
       int g3 = (int)std::min<int64_t>((nslots + 255) / 256, (int64_t)dev.sms * 8);
-      k_compact<<<g3, 256, 0, stream>>>(P, T, nslots, P.slot_bytes, G_n, 0, O);
+      k_compact<<<g3, 256, 0, stream>>>(P, T, nslots, P.slot_bytes, G_n, O);
     }
     ck(cudaGetLastError(), "compact launch");
     ck(cudaMemcpyAsync(host, counters, 4 * (4 + P.num_keys + P.num_outs), cudaMemcpyDeviceToHost, stream),

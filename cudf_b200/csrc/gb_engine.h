@@ -90,6 +90,7 @@ struct Options {
   // bound; a call whose flags show an overflow is redone with 1, which checks
   // after each stage and regrows tables as it goes
   int sync_checks = 0;
+  int full_sketch = 0;  // internal: 1 counts every row even where a sample shows few groups
 };
 
 // Option fields, as bits of Options::set_mask and TuningRule::mask.

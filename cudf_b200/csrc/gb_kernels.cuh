@@ -7,8 +7,9 @@
 //   k_var_pass       second pass of VARIANCE/STD
 //   k_finish_count   adds the all-ones-key slot to the group count
 //   k_compact        gathers occupied slots into dense key and result columns
-//   k_sketch         full-pass HyperLogLog + per-bucket row counts (group
-//                    estimate, partition region sizes)
+//   k_sketch         HyperLogLog + per-bucket row counts of all rows (group
+//                    estimate, partition region sizes) or of a sample
+//   k_sketch_few     whether the sample is enough (few groups)
 #pragma once
 #include <cub/block/block_scan.cuh>
 
@@ -356,34 +357,16 @@ __device__ __forceinline__ uint64_t finalize(const Plan& P, const OutSpec& o, co
   }
 }
 
-// Writes the occupied slots among [base, base + blockDim.x) of one table into
-// dense output columns (positions reserved per block on O.counters[2]).
-// Every thread of the block calls it (it synchronises the block).
-__device__ __forceinline__ void compact_block(const Plan& P, const uint8_t* T, int64_t nslots, int stride,
-                                              int64_t limit, int dense, const OutPtrs& O, int64_t base,
-                                              void* scan_storage, unsigned int* s_base)
+// Writes a slot's key and result columns at row `pos`.  Every lane of a warp
+// calls it (warp-wide mask assembly); its occupied lanes write consecutive rows.
+__device__ __forceinline__ void emit_slot(const Plan& P, const uint8_t* slot, bool occ, int64_t pos, const OutPtrs& O)
 {
-  using Scan = cub::BlockScan<int, 256>;
-  typename Scan::TempStorage& tmp = *(typename Scan::TempStorage*)scan_storage;
-  int64_t i = base + threadIdx.x;
-  const uint8_t* slot = T + i * (int64_t)stride;
-  bool occ = i < nslots && (dense || slot_occupied(P, slot, i == nslots - 1));
-  if (occ && !dense && i == nslots - 1) atomicAdd(O.counters + 3, 1u);
-  int local, total;
-  Scan(tmp).ExclusiveSum(occ ? 1 : 0, local, total);
-  if (threadIdx.x == 0) *s_base = total ? atomicAdd(O.counters + 2, (unsigned)total) : 0;
-  __syncthreads();
-  if (occ && (int64_t)*s_base + local >= limit) {
-    atomicOr(O.counters + 1, 1u);  // more occupied slots than counted groups
-    occ = false;
-  }
-  // every lane of the block runs what follows (warp-wide mask assembly)
-  const int64_t pos = (int64_t)*s_base + local;
   uint64_t w[2] = {0, 0};
   if (occ) {
     w[0] = ((const uint64_t*)slot)[0];
     w[1] = P.key_words == 2 ? ((const uint64_t*)slot)[1] : 0;
   }
+#pragma unroll 1
   for (int k = 0; k < P.num_keys; ++k) {
     const KeyCol& c = P.keys[k];
     const bool is_null = occ && c.has_null_bit && ((w[c.null_word] >> c.null_shift) & 1);
@@ -394,6 +377,7 @@ __device__ __forceinline__ void compact_block(const Plan& P, const uint8_t* T, i
     if (O.key_mask[k]) warp_mask_or(O.key_mask[k], occ, !is_null, pos);
     count_nulls(is_null, O.counters + 4 + k);
   }
+#pragma unroll 1
   for (int j = 0; j < P.num_outs; ++j) {
     const OutSpec& o = P.outs[j];
     bool valid = true;
@@ -405,23 +389,43 @@ __device__ __forceinline__ void compact_block(const Plan& P, const uint8_t* T, i
     if (O.out_mask[j]) warp_mask_or(O.out_mask[j], occ, valid, pos);
     count_nulls(occ && !valid, O.counters + 4 + P.num_keys + j);
   }
+}
+
+// Writes the occupied slots among [base, base + blockDim.x) of one table into
+// dense output columns (positions reserved per block on O.counters[2]).
+// Every thread of the block calls it (it synchronises the block).
+__device__ __forceinline__ void compact_block(const Plan& P, const uint8_t* T, int64_t nslots, int stride,
+                                              int64_t limit, const OutPtrs& O, int64_t base,
+                                              void* scan_storage, unsigned int* s_base)
+{
+  using Scan = cub::BlockScan<int, 256>;
+  typename Scan::TempStorage& tmp = *(typename Scan::TempStorage*)scan_storage;
+  int64_t i = base + threadIdx.x;
+  const uint8_t* slot = T + i * (int64_t)stride;
+  bool occ = i < nslots && slot_occupied(P, slot, i == nslots - 1);
+  if (occ && i == nslots - 1) atomicAdd(O.counters + 3, 1u);
+  int local, total;
+  Scan(tmp).ExclusiveSum(occ ? 1 : 0, local, total);
+  if (threadIdx.x == 0) *s_base = total ? atomicAdd(O.counters + 2, (unsigned)total) : 0;
+  __syncthreads();
+  if (occ && (int64_t)*s_base + local >= limit) {
+    atomicOr(O.counters + 1, 1u);  // more occupied slots than counted groups
+    occ = false;
+  }
+  emit_slot(P, slot, occ, (int64_t)*s_base + local, O);
   __syncthreads();
 }
 
-// nslots_dev (optional): a device count that bounds nslots (dense slots
-// written by the partitioned pass, read here instead of on the host).
 static __global__ void __launch_bounds__(256) k_compact(const __grid_constant__ Plan P, const uint8_t* T,
-                                                        int64_t nslots, int stride, int64_t limit, int dense,
-                                                        const __grid_constant__ OutPtrs O,
-                                                        const unsigned long long* nslots_dev = nullptr)
+                                                        int64_t nslots, int stride, int64_t limit,
+                                                        const __grid_constant__ OutPtrs O)
 {
   using Scan = cub::BlockScan<int, 256>;
   __shared__ typename Scan::TempStorage tmp;
   __shared__ unsigned int s_base;
-  if (nslots_dev) nslots = min(nslots, (int64_t)*(volatile const unsigned long long*)nslots_dev);
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < nslots; base += step)
-    compact_block(P, T, nslots, stride, limit, dense, O, base, &tmp, &s_base);
+    compact_block(P, T, nslots, stride, limit, O, base, &tmp, &s_base);
 }
 
 // ---- group-count estimate ----
@@ -440,31 +444,33 @@ inline size_t sketch_smem() { return ((size_t(1) << kHllBits) + (size_t(1) << kB
 
 // Keys other than one plain 64-bit column are packed four rows per thread; a
 // warp's rows are consecutive, its next step's lines on their way into L2.
-// While the keys of a warp repeat (few groups, or a hot key), rows of one
-// bucket are counted by one lane: 32 lanes adding to the same few counters
-// queue on them.
+//
+// chunks > 0: only that many runs of 128 rows, one from each of `chunks` equal
+// strata at a scrambled place (so that no period of the data can hide groups).
+// skip (optional): a device flag; set, the kernel leaves at once.
 static __global__ void __launch_bounds__(512) k_sketch(const __grid_constant__ Plan P, unsigned int* hll,
-                                                       unsigned int* buckets)
+                                                       unsigned int* buckets, int64_t chunks, const unsigned int* skip)
 {
   constexpr int NT = 512;
+  constexpr int SR = 4;
+  if (skip && *skip) return;
   extern __shared__ unsigned int sk[];
   unsigned int* reg = sk;
   unsigned int* bk = sk + (1 << kHllBits);
   for (int i = threadIdx.x; i < (1 << kHllBits) + (1 << kBucketBits); i += NT) sk[i] = 0;
   __syncthreads();
   const int64_t n = P.num_rows;
-  auto see = [&](uint64_t h) {  // registers only rise, and soon rarely: read before the atomic
+  auto rank_of = [](uint64_t h) {
     const uint64_t low = h << 24;
-    const unsigned rank = low ? (unsigned)__clzll((long long)low) + 1u : 41u;
-    unsigned int* r = &reg[(h >> 40) & ((1u << kHllBits) - 1)];
-    if (*(volatile unsigned int*)r < rank) atomicMax(r, rank);
+    return low ? (unsigned)__clzll((long long)low) + 1u : 41u;
   };
-  auto add = [&](uint64_t h) {
-    atomicAdd(&bk[h >> (64 - kBucketBits)], 1u);
-    see(h);
-  };
-  if (P.num_keys == 1 && !P.keys[0].mask && P.keys[0].width == 8 && P.keys[0].cat != CAT_F64) {
+  const bool plain = P.num_keys == 1 && !P.keys[0].mask && P.keys[0].width == 8 && P.keys[0].cat != CAT_F64;
+  if (plain && chunks == 0) {
     // one plain 64-bit key: four rows per thread in flight
+    auto add = [&](uint64_t h) {
+      atomicAdd(&bk[h >> (64 - kBucketBits)], 1u);
+      atomicMax(&reg[(h >> 40) & ((1u << kHllBits) - 1)], rank_of(h));
+    };
     const int64_t stride = (int64_t)gridDim.x * NT;
     const unsigned long long* kd = (const unsigned long long*)P.keys[0].data + P.keys[0].offset;
     int64_t row = blockIdx.x * (int64_t)NT + threadIdx.x;
@@ -477,7 +483,6 @@ static __global__ void __launch_bounds__(512) k_sketch(const __grid_constant__ P
     }
     for (; row < n; row += stride) add(fmix64(__ldg(kd + row)));
   } else {
-    constexpr int SR = 4;
     const int lane = threadIdx.x & 31;
     const int64_t step = (int64_t)gridDim.x * NT * SR;
     // a lane's line of the warp's step (32 SR rows of one key column)
@@ -493,32 +498,31 @@ static __global__ void __launch_bounds__(512) k_sketch(const __grid_constant__ P
       }
       left -= lines;
     }
-    bool repeats = false;
-    int since = 0;
-    for (int64_t w0 = (blockIdx.x * (int64_t)NT + (threadIdx.x & ~31)) * SR; w0 < n; w0 += step) {
-      if (line && w0 + step + 32 * SR <= n) asm volatile("prefetch.global.L2 [%0];" ::"l"(line + (w0 + step) * line_w));
+    // registers only rise, and soon rarely: read before the atomic (Zipf pairs
+    // 0.69 -> 0.63 ms; the plain key's loop above is faster without)
+    auto add = [&](uint64_t h) {
+      atomicAdd(&bk[h >> (64 - kBucketBits)], 1u);
+      unsigned int* r = &reg[(h >> 40) & ((1u << kHllBits) - 1)];
+      const unsigned rank = rank_of(h);
+      if (*(volatile unsigned int*)r < rank) atomicMax(r, rank);
+    };
+    const int64_t end = chunks > 0 ? chunks * 32 * SR : n;
+    for (int64_t i0 = (blockIdx.x * (int64_t)NT + (threadIdx.x & ~31)) * SR; i0 < end; i0 += step) {
+      int64_t w0 = i0;
+      if (chunks > 0) {
+        const int64_t stratum = n / chunks, s = i0 / (32 * SR);
+        w0 = s * stratum + (int64_t)(fmix64((uint64_t)s) % (uint64_t)(stratum - 32 * SR));
+      } else if (line && w0 + step + 32 * SR <= n) {
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(line + (w0 + step) * line_w));
+      }
       uint64_t k0[SR], k1[SR];
       bool live[SR];
 #pragma unroll
       for (int j = 0; j < SR; ++j) live[j] = w0 + lane + 32 * j < n;
       pack_rows<2, SR>(P, w0 + lane, k0, k1, live);
-      const bool look = (since++ & 15) == 0;
-      if (look) repeats = false;
 #pragma unroll
-      for (int j = 0; j < SR; ++j) {
-        const uint64_t h = hash_key(k0[j], k1[j], P.key_words);
-        if (repeats || look) {
-          const unsigned b = (unsigned)(h >> (64 - kBucketBits));
-          const unsigned peers = __match_any_sync(0xFFFFFFFFu, live[j] ? b : 0x80000000u);
-          if (look) repeats = repeats || __reduce_max_sync(0xFFFFFFFFu, live[j] ? (unsigned)__popc(peers) : 0u) >= 8;
-          if (live[j]) {
-            if (lane == __ffs(peers) - 1) atomicAdd(&bk[b], __popc(peers));
-            see(h);
-          }
-        } else if (live[j]) {
-          add(h);
-        }
-      }
+      for (int j = 0; j < SR; ++j)
+        if (live[j]) add(hash_key(k0[j], k1[j], P.key_words));
     }
   }
   __syncthreads();
@@ -526,6 +530,29 @@ static __global__ void __launch_bounds__(512) k_sketch(const __grid_constant__ P
     if (reg[i]) atomicMax(hll + i, reg[i]);
   for (int i = threadIdx.x; i < (1 << kBucketBits); i += NT)
     if (bk[i]) atomicAdd(buckets + i, bk[i]);
+}
+
+// Whether a sampled sketch can stand for the whole pass: at most 1024 buckets
+// in use, none seen fewer than 16 times, so groups the sample missed hold about
+// a millionth of the rows (their rows still find room, or are listed).  Then
+// *few is set and the sample's registers and buckets become the sketch's.
+static __global__ void __launch_bounds__(1024) k_sketch_few(const unsigned int* sample, unsigned int* sketch, unsigned int* few)
+{
+  const unsigned int* b = sample + (1 << kHllBits);
+  int used = 0;
+  bool rare = false;
+  for (int i = threadIdx.x; i < (1 << kBucketBits); i += 1024) {
+    used += b[i] > 0;
+    rare = rare || (b[i] > 0 && b[i] < 16);
+  }
+  __shared__ int s_used;
+  if (threadIdx.x == 0) s_used = 0;
+  const bool any = __syncthreads_or(rare);
+  atomicAdd(&s_used, used);
+  __syncthreads();
+  if (any || s_used > 1024 || s_used == 0) return;
+  for (int i = threadIdx.x; i < (1 << kHllBits) + (1 << kBucketBits); i += 1024) sketch[i] = sample[i];
+  if (threadIdx.x == 0) *few = 1;
 }
 
 }  // namespace gb

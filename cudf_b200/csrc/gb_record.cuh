@@ -696,8 +696,8 @@ __device__ __forceinline__ void apply_columns(const RecSpec& S, int nc, int rows
 template <int KW, int RW, bool WAGG>
 __global__ void __launch_bounds__(1024, 1) k_rec_aggregate(const __grid_constant__ Plan P,
                                                            const __grid_constant__ RecArgs A,
-                                                           const __grid_constant__ RecSpec S, TableRef G, DenseRef D,
-                                                           int scap, int sfill,
+                                                           const __grid_constant__ RecSpec S, TableRef G, EmitRef D,
+                                                           const __grid_constant__ OutPtrs O, int scap, int sfill,
                                                            const __grid_constant__ SlotTemplate tmpl)
 {
   constexpr int NT = 1024;
@@ -707,8 +707,8 @@ __global__ void __launch_bounds__(1024, 1) k_rec_aggregate(const __grid_constant
   using ScanT = cub::BlockScan<unsigned, NT>;
   __shared__ typename ScanT::TempStorage scan_tmp;
   __shared__ int s_part;
-  __shared__ unsigned int s_used, s_spill, s_new;
-  __shared__ unsigned long long s_base;
+  __shared__ unsigned int s_used, s_spill, s_new, s_base;
+  __shared__ unsigned int s_cnt[NT / 2];  // (16 rounds of NT slots, each at least 24 bytes, fill shared memory) x 32 warps
   if (threadIdx.x == 0) s_new = 0;
   const int stride = G.stride;
   const int nw = stride / 8;
@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(1024, 1) k_rec_aggregate(const __grid_constant
       apply_columns<R, RW, WAGG>(S, nc, rows_off, sa, vb, rec);
     }
     __syncthreads();
-    p2_flush<NT, ScanT>(P, G, D, slots, scap, s_spill != 0 || item.merge, scan_tmp, &s_base, &s_new);
+    p2_flush<NT, ScanT>(P, G, D, O, slots, scap, s_spill != 0 || item.merge, scan_tmp, s_cnt, &s_base, &s_new);
     __syncthreads();
   }
   if (threadIdx.x == 0 && s_new) atomicAdd(G.counters, s_new);

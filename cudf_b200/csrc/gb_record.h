@@ -80,10 +80,10 @@ bool record_layout(const Plan& P, RecSpec& S);
 bool launch_rec_scatter(const Plan& P, const RecArgs& A, const RecSpec& S, int smem_optin, cudaStream_t stream);
 // Pass 2 over A's items, for one- and two-word keys; `wagg`: rows of one slot
 // combined per warp first.
-void launch_rec_aggregate1(const Plan& P, const RecArgs& A, const RecSpec& S, const TableRef& G, const DenseRef& D,
-                           int scap, int sfill, const SlotTemplate& tmpl, bool wagg, cudaStream_t stream);
-void launch_rec_aggregate2(const Plan& P, const RecArgs& A, const RecSpec& S, const TableRef& G, const DenseRef& D,
-                           int scap, int sfill, const SlotTemplate& tmpl, bool wagg, cudaStream_t stream);
+void launch_rec_aggregate1(const Plan& P, const RecArgs& A, const RecSpec& S, const TableRef& G, const EmitRef& D,
+                           const OutPtrs& O, int scap, int sfill, const SlotTemplate& tmpl, bool wagg, cudaStream_t stream);
+void launch_rec_aggregate2(const Plan& P, const RecArgs& A, const RecSpec& S, const TableRef& G, const EmitRef& D,
+                           const OutPtrs& O, int scap, int sfill, const SlotTemplate& tmpl, bool wagg, cudaStream_t stream);
 // Applies the listed records to the global spill table.
 void launch_rec_spill(const Plan& P, const RecArgs& A, const RecSpec& S, const TableRef& G, int grid,
                       cudaStream_t stream);

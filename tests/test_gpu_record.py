@@ -115,3 +115,43 @@ def test_float32_sums_round_once(mode, n, groups):
         assert v.dtype == np.float32
         assert np.all(np.abs(v.astype(np.float64) - exact) <= np.spacing(exact.astype(np.float32)))
     assert np.allclose(res[0][1].to_numpy()[0], total / count, rtol=n * 2.0**-52, atol=0)
+
+
+def _fmix64(k):
+    k = k.astype(np.uint64)
+    with np.errstate(over="ignore"):
+        k ^= k >> np.uint64(33)
+        k *= np.uint64(0xff51afd7ed558ccd)
+        k ^= k >> np.uint64(33)
+        k *= np.uint64(0xc4ceb9fe1a85ec53)
+        k ^= k >> np.uint64(33)
+    return k
+
+
+@pytest.mark.parametrize("hidden", [0, 40, 70_000])
+@pytest.mark.parametrize("width", [1, 3])
+def test_sampled_sketch_with_groups_it_misses(hidden, width):
+    """Few groups on a large input are sized from a sample of 4096 runs of 128
+    rows.  Groups placed on rows that the sample does not visit still come out:
+    they find room in the shared tables, are listed, or (more than the list
+    holds) the call is redone from a pass over all rows."""
+    import cudf_b200 as cb
+    from cudf_b200 import aggregation as agg
+    n, chunks = (8 << 20) + 77, 4096
+    rng = np.random.default_rng(hidden + width)
+    key = rng.integers(0, 5, n).astype(np.int64)
+    stratum = n // chunks
+    s = np.arange(chunks, dtype=np.int64)
+    start = s * stratum + (_fmix64(s) % np.uint64(stratum - 128)).astype(np.int64)
+    seen = np.zeros(n, bool)
+    seen[(start[:, None] + np.arange(128)).ravel()] = True
+    rows = rng.permutation(np.nonzero(~seen)[0])[:hidden]
+    key[rows] = 1000 + np.arange(hidden)
+    v = rng.integers(-10**6, 10**6, n)
+    f = rng.normal(size=n)
+    reqs = [(cb.Column.from_numpy(v), [agg.sum(), agg.min(), agg.max(), agg.count()]),
+            (cb.Column.from_numpy(f, rng.random(n) > 0.1), [agg.sum(), agg.mean()]),
+            (cb.Column.from_numpy(f), [agg.max()])][:width]
+    gb, uk, *_ = run_both([cb.Column.from_numpy(key)], reqs)
+    assert uk.num_rows() == 5 + hidden
+    assert gb.stats()["mode"] == (1 if hidden < 70_000 else gb.stats()["mode"])
