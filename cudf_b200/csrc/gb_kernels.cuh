@@ -273,29 +273,25 @@ __device__ __forceinline__ void store_width(void* base, int64_t i, int width, ui
   }
 }
 
-__device__ __forceinline__ void count_nulls(bool is_null, unsigned int* counter)
-{
-  unsigned m = __ballot_sync(__activemask(), is_null);
-  if (m && (threadIdx.x & 31) == (__ffs(m) - 1)) atomicAdd(counter, __popc(m));
-}
-
-// Sets the validity bits of a warp's output rows.  The occupied lanes of a
-// warp write consecutive positions (pos of the lowest occupied lane, + 1 per
-// occupied lane), so their bits form one run: assembled with one warp OR
-// reduction and stored with at most two atomic ORs instead of one per row.
-// Every lane of the warp calls it.
-__device__ __forceinline__ void warp_mask_or(uint32_t* mask, bool occ, bool bit, int64_t pos)
+// Validity bits and null count of one column for a warp's output rows.  The
+// occupied lanes (occm, this lane's rank among them) write consecutive rows
+// from `pos0` on, so their bits form one run, stored by the lowest occupied
+// lane with at most two atomic ORs.  Every lane of the warp calls it.
+__device__ __forceinline__ void warp_validity(uint32_t* mask, unsigned int* nulls, unsigned occm, unsigned rank, bool bad,
+                                              int64_t pos0)
 {
   const unsigned full = 0xFFFFFFFFu;
-  const unsigned occm = __ballot_sync(full, occ);
-  if (!occm) return;
-  const int lane = threadIdx.x & 31;
-  const unsigned rank = __popc(occm & ((1u << lane) - 1));
-  const unsigned word = __reduce_or_sync(full, (occ && bit) ? (1u << rank) : 0u);
-  if (lane == __ffs(occm) - 1 && word) {
-    const int sh = (int)(pos & 31);
-    atomicOr(mask + (pos >> 5), word << sh);
-    if (sh && (word >> (32 - sh))) atomicOr(mask + (pos >> 5) + 1, word >> (32 - sh));
+  const unsigned badm = __ballot_sync(full, bad);
+  const bool lead = occm && (threadIdx.x & 31) == __ffs(occm) - 1;
+  if (badm && lead) atomicAdd(nulls, __popc(badm));
+  if (!mask) return;
+  const int n = __popc(occm);
+  unsigned word = n == 32 ? full : (1u << n) - 1u;
+  if (badm) word &= ~__reduce_or_sync(full, bad ? 1u << rank : 0u);
+  if (lead && word) {
+    const int sh = (int)(pos0 & 31);
+    atomicOr(mask + (pos0 >> 5), word << sh);
+    if (sh && (word >> (32 - sh))) atomicOr(mask + (pos0 >> 5) + 1, word >> (32 - sh));
   }
 }
 
@@ -361,6 +357,8 @@ __device__ __forceinline__ uint64_t finalize(const Plan& P, const OutSpec& o, co
 // calls it (warp-wide mask assembly); its occupied lanes write consecutive rows.
 __device__ __forceinline__ void emit_slot(const Plan& P, const uint8_t* slot, bool occ, int64_t pos, const OutPtrs& O)
 {
+  const unsigned occm = __ballot_sync(0xFFFFFFFFu, occ);
+  const unsigned rank = __popc(occm & ((1u << (threadIdx.x & 31)) - 1));
   uint64_t w[2] = {0, 0};
   if (occ) {
     w[0] = ((const uint64_t*)slot)[0];
@@ -374,20 +372,17 @@ __device__ __forceinline__ void emit_slot(const Plan& P, const uint8_t* slot, bo
       const uint64_t bits = c.width == 8 ? w[c.word] : (w[c.word] >> c.shift) & ((1ull << (8 * c.width)) - 1);
       store_width(O.key_data[k], pos, c.width, is_null ? 0 : bits);
     }
-    if (O.key_mask[k]) warp_mask_or(O.key_mask[k], occ, !is_null, pos);
-    count_nulls(is_null, O.counters + 4 + k);
+    if (O.key_mask[k]) warp_validity(O.key_mask[k], O.counters + 4 + k, occm, rank, is_null, pos);
   }
 #pragma unroll 1
   for (int j = 0; j < P.num_outs; ++j) {
     const OutSpec& o = P.outs[j];
     bool valid = true;
-    uint64_t bits = 0;
     if (occ) {
-      bits = finalize(P, o, slot, valid);
+      const uint64_t bits = finalize(P, o, slot, valid);
       store_width(O.out_data[j], pos, o.out_width, valid ? bits : 0);
     }
-    if (O.out_mask[j]) warp_mask_or(O.out_mask[j], occ, valid, pos);
-    count_nulls(occ && !valid, O.counters + 4 + P.num_keys + j);
+    warp_validity(O.out_mask[j], O.counters + 4 + P.num_keys + j, occm, rank, occ && !valid, pos);
   }
 }
 
