@@ -1101,10 +1101,20 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
     stage.rows_per_cta = ((n + dev.sms - 1) / dev.sms + 63) & ~(int64_t)63;
     // copies of the table: as many as fit, while each still sees enough rows
     // per group to be worth folding back
-    const int64_t slots = std::min<int64_t>(scap_rec, (2 * est + 16 + 3) & ~(int64_t)3);
-    const int64_t fit = scap_rec / slots, worth = stage.rows_per_cta / (16 * est);
+    // (an odd number of four-slot buckets and of 8- or 16-byte units per copy:
+    // see k_stage_aggregate)
+    const int64_t budget = (int64_t)scap_rec * (P.slot_bytes + 4);
+    const int64_t unit = 8 * P.key_words;
+    int64_t slots = std::min<int64_t>(scap_rec, (2 * est + 16 + 3) & ~(int64_t)3);
+    if ((slots / 4) % 2 == 0 && slots + 4 <= scap_rec) slots += 4;
+    auto pitch_of = [&](int64_t sl) {
+      const int64_t p = sl * P.slot_bytes;
+      return (p / unit) % 2 ? p : p + unit;
+    };
+    const int64_t fit = budget / (slots * 4 + pitch_of(slots)), worth = stage.rows_per_cta / (16 * est);
     stage.replicas = (int)std::max<int64_t>(1, std::min<int64_t>(kMaxReplicas, std::min(fit, worth)));
     stage.slots = (int)(stage.replicas == 1 ? std::min<int64_t>(scap_rec, (4 * est + 64 + 3) & ~(int64_t)3) : slots);
+    stage.pitch = (int)(stage.replicas == 1 ? (int64_t)stage.slots * P.slot_bytes : pitch_of(slots));
     stage.sfill = std::max(1, (int)(stage.slots * 0.9));
     // rows of one slot are folded per warp first where a key may hold a
     // sixteenth of the rows (two lanes of a warp) and the copies do not

@@ -21,7 +21,7 @@ int launch_stage(const Plan& P, const StageArgs& A, const TableRef& G, const Slo
   RecSpec S;
   stage_layout(P, S);
   const size_t total = (size_t)A.replicas * A.slots;
-  const size_t smem = total * 4 + (total + 1) * P.slot_bytes;
+  const size_t smem = total * 4 + (size_t)A.replicas * A.pitch + P.slot_bytes;
   const int grid = (int)((P.num_rows + A.rows_per_cta - 1) / A.rows_per_cta);
   auto go = [&](auto kern) {
     allow_max_smem((const void*)kern);

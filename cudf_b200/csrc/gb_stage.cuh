@@ -15,9 +15,12 @@ namespace gb {
 // table and thread t works on copy t mod replicas: with few groups the lanes of
 // a warp would otherwise queue on the same few slots, whose 64-bit and floating
 // reductions are compare-and-swap loops.  The copies are folded into the first
-// one at the end, and that one is merged into the global table.
-// Shared memory: per copy tags u32[slots], then per copy slots, then the
-// all-ones key's slot.
+// one at the end, and that one is merged into the global table.  The lanes of a
+// warp then meet the same slot of neighbouring copies, so the copies lie an odd
+// number of 8-byte units apart (16 for two-word keys): without that pad 60M rows
+// of six groups kept the shared-memory pipe 90% busy on bank conflicts.
+// Shared memory: per copy tags u32[slots], then per copy slots and pad, then
+// the all-ones key's slot.
 template <int KW, int MAXV, bool FOLD>
 __global__ void __launch_bounds__(1024, 1) k_stage_aggregate(const __grid_constant__ Plan P,
                                                              const __grid_constant__ StageArgs A,
@@ -33,22 +36,26 @@ __global__ void __launch_bounds__(1024, 1) k_stage_aggregate(const __grid_consta
   const int nw = stride / 8;
   const int total = A.replicas * A.slots;
   uint8_t* const slots = smem + (size_t)total * 4;
+  // slot i over all copies; slot `total` is the all-ones key's
+  auto slot_at = [&](int i) {
+    const int copy = i / A.slots;
+    return slots + (size_t)copy * A.pitch + (size_t)(i - copy * A.slots) * stride;
+  };
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
   auto table_of = [&](int copy) {
-    return RecTable{sbase + 4u * (uint32_t)(copy * A.slots), sbase + 4u * (uint32_t)total + (uint32_t)(copy * A.slots * stride),
+    return RecTable{sbase + 4u * (uint32_t)(copy * A.slots), sbase + 4u * (uint32_t)total + (uint32_t)(copy * A.pitch),
                     (uint32_t)A.slots / 4, stride, A.sfill, (uint32_t)__cvta_generic_to_shared(s_used + copy)};
   };
   for (int i = threadIdx.x; i < total / 4; i += NT) ((uint4*)smem)[i] = make_uint4(0, 0, 0, 0);
-  for (int w = 0; w < nw; ++w) {
-    const unsigned long long t = tmpl.w[w];
-    for (int s = threadIdx.x; s < total + (KW == 1); s += NT)
-      *(unsigned long long*)(slots + ((size_t)s * nw + w) * 8) = t;
+  for (int i = threadIdx.x; i < total + (KW == 1); i += NT) {
+    uint8_t* const s = slot_at(i);
+    for (int w = 0; w < nw; ++w) *(unsigned long long*)(s + w * 8) = tmpl.w[w];
   }
   for (int i = threadIdx.x; i < A.replicas; i += NT) s_used[i] = 0;
   if (threadIdx.x == 0) s_new = 0;
   __syncthreads();
   const RecTable table = table_of(threadIdx.x % A.replicas);
-  const uint32_t ones = sbase + 4u * (uint32_t)total + (uint32_t)(total * stride);
+  const uint32_t ones = sbase + 4u * (uint32_t)total + (uint32_t)(A.replicas * A.pitch);
   const int nc = S.ncols;
   const int lane = threadIdx.x & 31;
   const int64_t b = (int64_t)blockIdx.x * A.rows_per_cta;
@@ -117,7 +124,7 @@ __global__ void __launch_bounds__(1024, 1) k_stage_aggregate(const __grid_consta
   // the other copies into the first
   const RecTable first = table_of(0);
   for (int i = A.slots + threadIdx.x; i < total; i += NT) {
-    const uint8_t* s = slots + (size_t)i * stride;
+    const uint8_t* s = slot_at(i);
     if (!slot_occupied(P, s, false)) continue;
     const uint64_t w0 = ((const uint64_t*)s)[0], w1 = KW == 2 ? ((const uint64_t*)s)[1] : 0;
     const uint32_t d = rec_slot<KW>(first, w0, w1, hash_key(w0, w1, KW));
@@ -130,7 +137,7 @@ __global__ void __launch_bounds__(1024, 1) k_stage_aggregate(const __grid_consta
     if (slot_occupied(P, s, false)) merge_slot(P, G, s, &s_new);
   }
   if (KW == 1 && threadIdx.x == 0) {
-    const uint8_t* s = slots + (size_t)total * stride;
+    const uint8_t* s = slot_at(total);
     if (*(const uint32_t*)(s + P.rows_off) > 0) merge_slot(P, G, s, &s_new);
   }
   __syncthreads();

@@ -8,6 +8,7 @@ struct StageArgs {
   int64_t rows_per_cta;    // contiguous row range of a CTA (a multiple of 64)
   int32_t replicas;        // copies of the table in a CTA
   int32_t slots;           // slots of one copy (a multiple of four)
+  int32_t pitch;           // bytes from one copy's slots to the next one's
   int32_t sfill;           // slots of one copy that may be claimed
   int64_t* spill_rows;     // rows that fitted no copy
   unsigned int spill_cap;
