@@ -50,11 +50,11 @@ KERNELS_BY_MODE = {0: "k_aggregate<false>", 1: "k_aggregate<true>",
 # of a smaller case of the same workload scaled up; the capture command and
 # the per-kernel figures are in profiles/.
 # Mode 2: (bytes per row, bytes per group); the partitioned copy is written
-# and read once, and the dense slots are written once per group.
-TRAFFIC_MODEL = {2: (84.93, 75.1)}
+# and read once, and the result columns are written once per group.
+TRAFFIC_MODEL = {2: (90.43, 102.0)}
 TRAFFIC_SOURCE = {2: "ncu dram__bytes_read.sum + dram__bytes_write.sum of both kernels on the 20M-row "
-                     "case, scaled by rows (and by groups for the dense-slot writes); "
-                     "profiles/k_part_scatter_bulk_k_part_aggregate_20M.md"}
+                     "case, scaled by rows (and by groups for the result writes); "
+                     "profiles/k_rec_scatter_k_rec_aggregate_20M.md"}
 
 
 def algorithmic_bytes(n_rows: int, n_groups: int) -> tuple[float, float]:
