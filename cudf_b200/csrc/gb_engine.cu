@@ -632,7 +632,7 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   const bool sketch = opt.groups_hint < 0 && n > 65536;
   // From 8M rows on a sample of 512Ki rows is looked at first: with few groups
   // it is the sketch (60M rows of six groups: 0.31 ms for all of them), else it
-  // costs about 12 us ahead of the pass over all rows (0.1 to 0.7 ms).
+  // costs about 16 us ahead of the pass over all rows (0.1 to 0.6 ms).
   constexpr int64_t kSampleFrom = 8 << 20, kSampleChunks = 4096;
   const bool sample = sketch && !opt.full_sketch && n >= kSampleFrom;
   const size_t sketch_bytes = (sketch ? sketch_smem() : 0) * (sample ? 2 : 1) + (sketch ? 64 : 0);

@@ -91,9 +91,10 @@ __device__ __forceinline__ int p2_claim(unsigned int* work, uint8_t* smem, int s
 // all-ones key's slot (one-word keys; it cannot be told from an empty slot)
 // is always merged into the global table's dedicated slot.
 // The rows are written column by column with consecutive lanes on consecutive
-// rows: copying the slots out as they are (88 bytes apart per lane) makes one
-// store request per slot word, at 40 G requests a second 1.9 ms for 25M groups
-// of 24 bytes, and needs a compaction pass over the copy.
+// rows.  Against copying the slots out and compacting them afterwards: pass 2
+// 2.09 -> 2.23 ms at 1M groups (the compaction took 0.09), 3.52 -> 3.58 at 7.8M
+// (0.28), 1.98 -> 1.92 at 25M (0.53).  Out of line it was slower still (2.32 at
+// 1M): the plan's fields are then read through generic addresses.
 template <int NT, typename ScanT>
 __device__ __forceinline__ void p2_flush(const Plan& P2, const TableRef& G, const EmitRef& D, const OutPtrs& O,
                                          const uint8_t* smem, int scap, bool spilled,
