@@ -484,7 +484,7 @@ uint32_t* pinned()
 // finishes with a stream synchronisation, so the copy out of it is done before
 // the thread's next call writes it again.
 thread_local int64_t* t_regions = nullptr;
-constexpr size_t kRegionWords = 3 * 8192;
+constexpr size_t kRegionWords = 3 * kMaxParts;
 int64_t* pinned_regions()
 {
   if (!t_regions) ck(cudaMallocHost((void**)&t_regions, kRegionWords * 8), "cudaMallocHost");
@@ -742,7 +742,6 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   // whose partitions hold equally many buckets, at most 8192 (the scatter
   // keeps 12 B per partition in shared memory); beyond ~85% of that capacity
   // the shared tables would spill most groups and the global table is faster.
-  constexpr int kMaxParts = 8192;
   int nparts = 0;
   if (part_ok) {
     const int64_t sms = dev.sms;
@@ -766,6 +765,9 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   else mode = 0;
   if (mode == 1 && scap < 16) mode = 0;
   if (mode == 2 && !part_ok) mode = 0;
+  RecSpec rec;
+  if (mode == 2 && !(record_layout(P, rec) && rec_shape(P.key_words, rec.words, nparts, rec.nmask, dev.smem_optin).threads))
+    mode = 0;  // (every record size has a shape up to kMaxParts partitions)
 
   if (sampled && mode != 1) {  // only the shared stage does without every row's count
     Options o2 = opt_in;
@@ -925,8 +927,6 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
       std::memcpy(st3 + 2 * nparts, pbase.data(), 8 * nparts);
       ck(cudaMemcpyAsync(d_base, st3, 24 * (size_t)nparts, cudaMemcpyHostToDevice, stream), "h2d");
     }
-    RecSpec rec;
-    if (!record_layout(P, rec)) throw Error(ERR_LOGIC, "internal error: plan without a record layout");
     RecArgs A;
     std::memset(&A, 0, sizeof(A));
     A.nparts = nparts;

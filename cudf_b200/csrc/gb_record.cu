@@ -44,8 +44,7 @@ bool record_layout(const Plan& P, RecSpec& S)
   for (int v = 0; v < P.num_vals; ++v) order[v] = v;
   std::stable_sort(order, order + P.num_vals, [&](int a, int b) { return P.vals[a].width > P.vals[b].width; });
   int at[kMaxRecCols];
-  const int sizes[] = {2, 4, 6, 8, 12};
-  for (int words : sizes) {
+  for (int words : kRecSizes) {
     bool used[8 * kMaxRecWords] = {};
     for (int i = 0; i < key_bytes; ++i) used[i] = true;
     if (S.has_bits) used[8 * words - 1] = true;
@@ -91,12 +90,11 @@ bool record_layout(const Plan& P, RecSpec& S)
 
 namespace {
 template <int KW, int NT, int RPT, int MINB>
-bool launch(const Plan& P, const RecArgs& A, const RecSpec& S, int smem_optin, cudaStream_t stream)
+void launch(const Plan& P, const RecArgs& A, const RecSpec& S, cudaStream_t stream)
 {
-  const size_t T = (size_t)NT * RPT;
-  const size_t smem = T * S.words * 8 + (size_t)A.nparts * 8 + (size_t)S.nmask * (T / 32 + 1) * 4;
-  if ((smem + 2048) * MINB > (size_t)smem_optin) return false;
-  const int64_t ntiles = (P.num_rows + (int64_t)T - 1) / (int64_t)T;
+  constexpr int T = NT * RPT;
+  const size_t smem = rec_scatter_smem(T, S.words, A.nparts, S.nmask);
+  const int64_t ntiles = (P.num_rows + T - 1) / T;
   auto go = [&](auto kern) {
     allow_max_smem((const void*)kern);
     const int grid = (int)std::min<int64_t>(grid_for((const void*)kern, NT, smem, MINB), ntiles);
@@ -107,32 +105,37 @@ bool launch(const Plan& P, const RecArgs& A, const RecSpec& S, int smem_optin, c
   if (per <= 2) go(k_rec_scatter<KW, NT, RPT, MINB, 2>);
   else if (per <= 8) go(k_rec_scatter<KW, NT, RPT, MINB, 8>);
   else go(k_rec_scatter<KW, NT, RPT, MINB, 1>);
-  return true;
+}
+template <int KW, int NT, int MINB>
+bool launch_rows(int rows, const Plan& P, const RecArgs& A, const RecSpec& S, cudaStream_t s)
+{
+  switch (rows) {
+    case 8:
+      if constexpr (KW == 1) {
+        launch<KW, NT, 8, MINB>(P, A, S, s);
+        return true;
+      }
+      return false;
+    case 6: launch<KW, NT, 6, MINB>(P, A, S, s); return true;
+    case 5: launch<KW, NT, 5, MINB>(P, A, S, s); return true;
+    case 4: launch<KW, NT, 4, MINB>(P, A, S, s); return true;
+    case 3: launch<KW, NT, 3, MINB>(P, A, S, s); return true;
+    case 2: launch<KW, NT, 2, MINB>(P, A, S, s); return true;
+    case 1: launch<KW, NT, 1, MINB>(P, A, S, s); return true;
+    default: return false;
+  }
 }
 template <int KW>
-bool pick(const Plan& P, const RecArgs& A, const RecSpec& S, int o, cudaStream_t s)
+bool launch_shape(const RecShape& r, const Plan& P, const RecArgs& A, const RecSpec& S, cudaStream_t s)
 {
-  // Two CTAs per SM on the largest tile of which two fit, so that one loads
-  // while the other reserves or writes.  With less than two rows per partition
-  // in such a tile (thousands of partitions) one CTA on a tile as large as
-  // shared memory instead: 40M 16-byte rows over 4096 partitions take 0.68 ms
-  // against 0.85, 100M 32-byte rows over 740 partitions 1.63 against 1.58.
-  if (A.nparts > 6144 / S.words) {  // two CTAs of T rows hold about 12,288 words each
-    if constexpr (KW == 1)
-      if (launch<KW, 1024, 8, 1>(P, A, S, o, s)) return true;
-    if (launch<KW, 1024, 6, 1>(P, A, S, o, s) || launch<KW, 1024, 5, 1>(P, A, S, o, s)) return true;
-  }
-  if constexpr (KW == 1)
-    if (launch<KW, 512, 8, 2>(P, A, S, o, s)) return true;
-  return launch<KW, 512, 6, 2>(P, A, S, o, s) || launch<KW, 512, 5, 2>(P, A, S, o, s) ||
-         launch<KW, 512, 4, 2>(P, A, S, o, s) || launch<KW, 512, 3, 2>(P, A, S, o, s) ||
-         launch<KW, 512, 2, 2>(P, A, S, o, s) || launch<KW, 512, 1, 2>(P, A, S, o, s);
+  return r.ctas == 1 ? launch_rows<KW, 1024, 1>(r.rows, P, A, S, s) : launch_rows<KW, 512, 2>(r.rows, P, A, S, s);
 }
 }  // namespace
 
 bool launch_rec_scatter(const Plan& P, const RecArgs& A, const RecSpec& S, int smem_optin, cudaStream_t stream)
 {
-  return P.key_words == 1 ? pick<1>(P, A, S, smem_optin, stream) : pick<2>(P, A, S, smem_optin, stream);
+  const RecShape r = rec_shape(P.key_words, S.words, A.nparts, S.nmask, smem_optin);
+  return P.key_words == 1 ? launch_shape<1>(r, P, A, S, stream) : launch_shape<2>(r, P, A, S, stream);
 }
 
 void launch_rec_spill(const Plan& P, const RecArgs& A, const RecSpec& S, const TableRef& G, int grid,

@@ -8,6 +8,7 @@
 #include "gb_kernels.cuh"
 #include "gb_partition.cuh"
 #include "gb_plan.h"
+#include "gb_record_shape.h"
 
 namespace gb {
 
@@ -76,7 +77,7 @@ RecCol rec_col(const ValCol& c, int bit, int shift, int adv);
 // Lays the record out; false when the plan has no record form (more than
 // kMaxRecCols value columns).
 bool record_layout(const Plan& P, RecSpec& S);
-// Pass 1 over nparts partitions; false when no launch shape fits.
+// Pass 1 over nparts partitions; false when no launch shape fits (see rec_shape).
 bool launch_rec_scatter(const Plan& P, const RecArgs& A, const RecSpec& S, int smem_optin, cudaStream_t stream);
 // Pass 2 over A's items, for one- and two-word keys; `wagg`: rows of one slot
 // combined per warp first.
