@@ -932,7 +932,8 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
     A.nparts = nparts;
     A.end = d_end;
     A.cursor = d_cur;
-    A.recs = (uint64_t*)S.get((size_t)total * 8 * rec.words);
+    // 32-byte loads of records: the allocator gives 16-byte alignment only
+    A.recs = (uint64_t*)(((uintptr_t)S.get((size_t)total * 8 * rec.words + 16) + 31) & ~(uintptr_t)31);
     A.counters = counters;
     mark("partition scratch");
     if (opt.profile) ck(cudaEventRecord(events()[0], stream), "event");

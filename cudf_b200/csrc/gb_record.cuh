@@ -29,8 +29,9 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* p, unsigned bytes)
 }
 
 // ---- record loads ------------------------------------------------
-// A record starts on a multiple of its size up to 32 bytes (of 16 for the
-// 48-byte form), so it moves as 32-, 16- or 8-byte vectors.
+// The record array starts on a multiple of 32 bytes, so a record starts on a
+// multiple of 16, and where its size is a multiple of 32 on one of 32: it moves
+// as 16- or 32-byte vectors.
 template <int RW>
 __device__ __forceinline__ void rec_load(const uint64_t* p, uint64_t (&w)[RW])
 {

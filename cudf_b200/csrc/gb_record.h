@@ -62,7 +62,7 @@ struct RecArgs {
   int32_t nparts;
   const int64_t* end;            // [nparts] one past the last record of each region
   unsigned long long* cursor;    // [nparts] next free record of each region
-  uint64_t* recs;
+  uint64_t* recs;                // 32-byte aligned
   unsigned int* counters;        // [5] region overflow, [12] spill list length, [13] its overflow
   int64_t* spill_rows;           // pass 2: records that did not fit their shared table
   unsigned int spill_cap;
