@@ -134,10 +134,12 @@ struct Scratch {
         return;
       }
   }
-  ~Scratch()
+  void clear()
   {
     for (auto& b : bufs) A.deallocate(A.ctx, b.p, b.n, (void*)s);
+    bufs.clear();
   }
+  ~Scratch() { clear(); }
 };
 
 void Result::release()
@@ -592,8 +594,15 @@ int apply_tuning_rules(Options& o, int64_t rows, int64_t groups, int key_words, 
   return -1;
 }
 
-Result aggregate(const std::vector<Column>& keys, int null_policy, const std::vector<Request>& reqs,
-                 cudaStream_t stream, const Allocator& alloc, const Options& opt_in, Stats* stats)
+namespace {
+// What a call that throws leaves behind.
+struct CallState {
+  bool staged = false;       // copies out of the thread's pinned staging were queued
+  bool partitioned = false;  // the partitioned path was entered
+};
+
+Result aggregate_call(const std::vector<Column>& keys, int null_policy, const std::vector<Request>& reqs,
+                      cudaStream_t stream, const Allocator& alloc, const Options& opt_in, Stats* stats, CallState& state)
 {
   Options opt = opt_in;  // tuning rules may adjust it once the group estimate is known
   Plan P;
@@ -764,7 +773,7 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   else if (part_ok && part_fits && n >= (1 << 20) && est > smem_max) mode = 2;
   else mode = 0;
   if (mode == 1 && scap < 16) mode = 0;
-  if (mode == 2 && !part_ok) mode = 0;
+  if (mode == 2 && !(part_ok && opt.partition)) mode = 0;
   RecSpec rec;
   if (mode == 2 && !(record_layout(P, rec) && rec_shape(P.key_words, rec.words, nparts, rec.nmask, dev.smem_optin).threads))
     mode = 0;  // (every record size has a shape up to kMaxParts partitions)
@@ -772,7 +781,8 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   if (sampled && mode != 1) {  // only the shared stage does without every row's count
     Options o2 = opt_in;
     o2.full_sketch = 1;
-    return aggregate(keys, null_policy, reqs, stream, alloc, o2, stats);
+    S.clear();
+    return aggregate_call(keys, null_policy, reqs, stream, alloc, o2, stats, state);
   }
 
   // region sizes of the partitioned path: exact rows per partition from the
@@ -913,6 +923,7 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
 
   if (mode == 2) {
     // ---- pass 1: scatter rows into hash partitions ----
+    state.partitioned = true;
     int64_t total = pend.back();
     // region starts, ends and cursors (= starts): one pinned staging copy
     // into one device block
@@ -922,6 +933,7 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
     {
       if ((size_t)3 * nparts > kRegionWords) throw Error(ERR_LOGIC, "internal error: too many partitions");
       int64_t* st3 = pinned_regions();
+      state.staged = true;
       std::memcpy(st3, pbase.data(), 8 * nparts);
       std::memcpy(st3 + nparts, pend.data(), 8 * nparts);
       std::memcpy(st3 + 2 * nparts, pbase.data(), 8 * nparts);
@@ -1223,7 +1235,8 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
         Options o2 = opt_in;
         o2.sync_checks = 1;
         o2.full_sketch = 1;
-        return aggregate(keys, null_policy, reqs, stream, alloc, o2, stats);
+        S.clear();
+        return aggregate_call(keys, null_policy, reqs, stream, alloc, o2, stats, state);
       }
       const int64_t dn = mode == 2 ? (int64_t)(host[10] | ((uint64_t)host[11] << 32)) : 0;
       G_n = (int64_t)chost[2];
@@ -1258,6 +1271,27 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
   }
   if (stats) *stats = st;
   undo.keep = true;
+  return R;
+}
+}  // namespace
+
+Result aggregate(const std::vector<Column>& keys, int null_policy, const std::vector<Request>& reqs,
+                 cudaStream_t stream, const Allocator& alloc, const Options& opt, Stats* stats)
+{
+  CallState state;
+  try {
+    return aggregate_call(keys, null_policy, reqs, stream, alloc, opt, stats, state);
+  } catch (const Error& e) {
+    // the thread's next call writes its pinned staging again
+    if (state.staged) cudaStreamSynchronize(stream);
+    // rows as records can take up to about twice the columns' bytes: without
+    // room for them the global table, which needs no copy of the rows
+    if (e.code != ERR_ALLOC || !state.partitioned) throw;
+  }
+  Options o2 = opt;
+  o2.partition = 0;
+  Result R = aggregate_call(keys, null_policy, reqs, stream, alloc, o2, stats, state);
+  if (stats) ++stats->retries;
   return R;
 }
 

@@ -90,6 +90,7 @@ struct Options {
   // bound; a call whose flags show an overflow is redone with 1, which checks
   // after each stage and regrows tables as it goes
   int sync_checks = 0;
+  int partition = 1;    // internal: 0 keeps a call off the partitioned path (its scratch did not fit)
   int full_sketch = 0;  // internal: 1 counts every row even where a sample shows few groups
 };
 

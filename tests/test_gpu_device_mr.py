@@ -41,3 +41,45 @@ def test_blocks_aligned_to_16_bytes_are_enough(mode, two_words, kinds):
     _check(keys, reqs, uk, res)
     del uk, res
     assert not mr.live
+
+
+@pytest.mark.parametrize("tuning", [{}, {"force_mode": 2}])
+def test_rows_that_do_not_fit_as_records_take_the_global_table(tuning):
+    """32-byte records of 1.1M rows are 35 MB: a resource that gives 20 MB blocks holds every column
+    and the 50k groups' table, so the call still runs."""
+    import cudf_b200 as cb
+    from cudf_b200 import aggregation as agg
+    rng = np.random.default_rng(3)
+    n = 1_100_000
+    keys = [cb.Column.from_numpy(rng.integers(0, 50_000, n))]
+    reqs = [cb.GroupByRequest(cb.Column.from_numpy(rng.integers(-9, 9, n), rng.random(n) > 0.1), [agg.sum(), agg.max()])]
+    reqs.append(cb.GroupByRequest(cb.Column.from_numpy(rng.normal(size=n)), [agg.sum()]))
+    gb = cb.GroupBy(cb.Table(keys))
+    if tuning:
+        gb.set_tuning(**tuning)
+    mr = DeviceResource(limit=20_000_000)
+    uk, res = aggregate_with(gb, reqs, mr)
+    assert mr.refused and gb.stats()["mode"] == 0 and gb.stats()["retries"] == 1
+    _check(keys, reqs, uk, res)
+    del uk, res
+    assert not mr.live
+
+
+def test_a_call_that_fails_for_memory_leaves_the_next_one_alone():
+    """The blocks of a failed call go back, and the thread's next call, on another stream, gives its own result."""
+    import cudf_b200 as cb
+    from cudf_b200 import aggregation as agg
+    rng = np.random.default_rng(4)
+    n = 1_100_000
+    keys = [cb.Column.from_numpy(rng.integers(0, 50_000, n))]
+    reqs = [cb.GroupByRequest(cb.Column.from_numpy(rng.integers(-9, 9, n)), [agg.sum(), agg.max()])]
+    gb = cb.GroupBy(cb.Table(keys))
+    other = torch.cuda.Stream()
+    other.wait_stream(torch.cuda.current_stream())
+    for limit in (200_000, 1_000_000):
+        small = DeviceResource(limit=limit)
+        with pytest.raises(MemoryError):
+            aggregate_with(gb, reqs, small)
+        assert not small.live
+        uk, res = aggregate_with(gb, reqs, DeviceResource(), stream=other)
+        _check(keys, reqs, uk, res)
