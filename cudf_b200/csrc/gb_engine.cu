@@ -872,6 +872,14 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
   uint64_t cap = next_pow2((uint64_t)std::max<double>(1024.0, std::ceil((double)est / opt.load_factor)));
   cap = std::min<uint64_t>(cap, next_pow2((uint64_t)(2 * n + 2)));
   cap = std::max<uint64_t>(cap, 1024);
+  // a sample can miss the groups of a stretch of rows between two of its runs
+  // (sorted or clustered rows): room for as many as two strata or the list of
+  // unplaced rows hold, so that they do not cost a second pass
+  constexpr uint32_t kStageSpill = 1u << 16;
+  if (sampled) {
+    const uint64_t missed = std::min<uint64_t>(kStageSpill, 2 * (uint64_t)(n / kSampleChunks));
+    cap = std::max<uint64_t>(cap, next_pow2(missed + 2 * (uint64_t)est));
+  }
 
   uint8_t* T = nullptr;
   TableRef G{};
@@ -1167,7 +1175,7 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
     uint32_t top = 0;
     for (int b = 0; buckets && b < kNumBuckets; ++b) top = std::max(top, buckets[b]);
     stage_fold = stage.replicas < 32 && (!buckets || (int64_t)top * 16 > nsamp);
-    stage.spill_cap = 1u << 16;
+    stage.spill_cap = kStageSpill;
     stage.spill_rows = (int64_t*)S.get(sizeof(int64_t) * stage.spill_cap);
     stage.counters = counters;
   }
@@ -1259,13 +1267,14 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
     mark("compaction (synced)");
     if (deferred) {
       // an overflow anywhere (a table, a region, the result rows, a spill
-      // list): redo the call with checks after every stage
+      // list): redo the call with checks after every stage, or, where only a
+      // sample had sized it, from the count of every row
       const bool again = host[1] || chost[1] || (mode == 2 && (host[5] || host[13])) ||
                          (raw_stage && host[13]);
       if (again) {
         R.release();
         Options o2 = opt_in;
-        o2.sync_checks = 1;
+        o2.sync_checks = !sampled;
         o2.full_sketch = 1;
         S.clear();
         return aggregate_call(keys, null_policy, reqs, stream, alloc, o2, stats, state);

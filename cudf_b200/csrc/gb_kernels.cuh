@@ -528,9 +528,13 @@ static __global__ void __launch_bounds__(512) k_sketch(const __grid_constant__ P
 }
 
 // Whether a sampled sketch can stand for the whole pass: at most 1024 buckets
-// in use, none seen fewer than 16 times, so groups the sample missed hold about
-// a millionth of the rows (their rows still find room, or are listed).  Then
-// *few is set and the sample's registers and buckets become the sketch's.
+// in use, none seen fewer than 16 times.  Of rows in random order, groups that
+// the sample missed then hold about a millionth.  Of sorted or clustered rows
+// any stretch between two sampled runs (up to two strata less 128 rows, a
+// 2048th of all) and the last n mod chunks rows can hold groups of their own.
+// Either way their rows find room, are listed, or the call is redone from the
+// full pass.  Then *few is set and the sample's registers and buckets become
+// the sketch's.
 static __global__ void __launch_bounds__(1024) k_sketch_few(const unsigned int* sample, unsigned int* sketch, unsigned int* few)
 {
   const unsigned int* b = sample + (1 << kHllBits);
