@@ -799,10 +799,22 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
     else nparts = (int)std::min<uint64_t>(kMaxParts, next_pow2((uint64_t)tight));
   }
   const bool part_fits = (double)est <= 0.85 * (double)kMaxParts * sfill2;
+  // VARIANCE/STD look every group up in the global table in their second pass,
+  // so partitions only save updates: worth a copy of the rows from a few million
+  // of them on, sooner with several accumulators a row than with one or two, and
+  // not where groups have only a few rows.  Global table / partitioned in ms,
+  // one accumulator: 1.1M rows, 50K groups 0.19 / 0.24; 4M, 200K 0.35 / 0.36;
+  // 8M, 500K 0.67 / 0.58; 8M, 4M 1.31 / 1.49; 40M, 20M 9.1 / 10.0.  Four: 1.1M,
+  // 50K 0.27 / 0.28; 2M, 5K 0.31 / 0.42; 2M, 200K 0.36 / 0.35; 2M, 1M 0.61 / 0.69;
+  // 4M, 5K 0.47 / 0.43; 4M, 200K 0.54 / 0.46; 8M, 4M 2.96 / 2.51.
+  bool part_pays = true;
+  if (P.need_second_pass)
+    part_pays = P.num_accs > 2 ? n >= 3500000 || (n >= 2000000 && est >= 128 * (int64_t)dev.sms && n >= 4 * est)
+                               : n >= 6000000 && n >= 5 * est;
   int mode;
   if (opt.force_mode >= 0) mode = opt.force_mode;
   else if (scap >= 64 && est <= smem_max) mode = 1;
-  else if (part_ok && part_fits && n >= (1 << 20) && est > smem_max) mode = 2;
+  else if (part_ok && part_fits && part_pays && n >= (1 << 20) && est > smem_max) mode = 2;
   else mode = 0;
   if (mode == 1 && scap < 16) mode = 0;
   if (mode == 2 && !(part_ok && opt.partition)) mode = 0;
@@ -1060,7 +1072,8 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
     // spill list: room for the rows of the groups expected to spill
     uint32_t spill_list = (uint32_t)std::min<uint64_t>(
       1ull << 31, next_pow2((uint64_t)std::max<double>(262144.0, 4.0 * expect_spill)));
-    int64_t dcap = (int64_t)(est * 1.5) + (int64_t)nparts * 256 + 4096;
+    // rows that pass 2 writes itself (VARIANCE/STD: none, every group goes to T)
+    const int64_t dcap = P.need_second_pass ? 0 : (int64_t)(est * 1.5) + (int64_t)nparts * 256 + 4096;
     for (int attempt = 0;; ++attempt) {
       T = (uint8_t*)S.get((size_t)(spill_cap + 1) * P.slot_bytes);
       A.spill_rows = (int64_t*)S.get((size_t)spill_list * sizeof(int64_t));
