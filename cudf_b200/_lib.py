@@ -142,6 +142,8 @@ SIGNATURES = {
     "gb_batch_destroy": (None, [ctypes.c_void_p]),
     "gb_batch_set_tuning": (ctypes.c_int, [ctypes.POINTER(GbBatchRule), ctypes.c_int32,
                                            ctypes.POINTER(GbBatchLaunch)]),
+    "gb_batch_set_default_tuning": (ctypes.c_int, [ctypes.POINTER(GbBatchRule), ctypes.c_int32,
+                                                   ctypes.POINTER(GbBatchLaunch)]),
     "gb_server_create": (ctypes.c_int, [ctypes.POINTER(GbServerOptions), ctypes.POINTER(ctypes.c_void_p)]),
     "gb_server_submit": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(GbColumn), ctypes.c_int32, ctypes.c_int32,
                                         ctypes.POINTER(GbRequest), ctypes.c_int32, ctypes.POINTER(ctypes.c_int64)]),

@@ -84,15 +84,17 @@ def load(path: str = TUNING_FILE) -> List[Dict]:
     rules = d["rules"]
     set_rules(rules)
     if "batch" in d:
-        set_batch_tuning(d["batch"].get("rules", []), d["batch"].get("launch"))
+        # the shipped settings are defaults: small batches still get smaller tiles
+        set_batch_tuning(d["batch"].get("rules", []), d["batch"].get("launch"), default=path == TUNING_FILE)
     return rules
 
 
 # -- batched launches (gb_batch_set_tuning) -------------------------------------
-def set_batch_tuning(rules: Sequence[Dict], launch: Optional[Dict] = None) -> None:
+def set_batch_tuning(rules: Sequence[Dict], launch: Optional[Dict] = None, default: bool = False) -> None:
     """Installs batch tuning: launch {"block", "tile_rows", "smem_bytes"} and
     per-instance rules [{"max_rows", "max_groups", "smem_slots", "headroom_pct"}]
-    (first match applies; -1 / 0 leave a field unset)."""
+    (first match applies; -1 / 0 leave a field unset).  With `default` the
+    launch's tile_rows holds for large batches and smaller ones take fewer."""
     arr = (_lib.GbBatchRule * max(1, len(rules)))()
     for i, r in enumerate(rules):
         arr[i] = _lib.GbBatchRule(int(r["max_rows"]), int(r["max_groups"]), int(r.get("smem_slots", -1)),
@@ -101,7 +103,8 @@ def set_batch_tuning(rules: Sequence[Dict], launch: Optional[Dict] = None) -> No
     if launch:
         lp = ctypes.byref(_lib.GbBatchLaunch(int(launch["block"]), int(launch["tile_rows"]),
                                              int(launch["smem_bytes"])))
-    _lib.check(_lib.lib().gb_batch_set_tuning(arr, len(rules), lp))
+    install = _lib.lib().gb_batch_set_default_tuning if default else _lib.lib().gb_batch_set_tuning
+    _lib.check(install(arr, len(rules), lp))
 
 
 BATCH_LAUNCH_DEFAULT = {"block": 512, "tile_rows": 65536, "smem_bytes": 160 * 1024}

@@ -698,13 +698,15 @@ void Batch::prepare(const std::vector<std::vector<Column>>& keys, int null_polic
   }
   B.d_counters.get(A, (size_t)ninst * B.counter_words * 4, stream);
   B.d_work.get(A, 16, stream);
-  // tiles: instances cut into tile_rows-row pieces, largest first; smaller
-  // batches into smaller pieces, so that the SMs still share them evenly (12M
-  // rows in 64Ki-row tiles are 183 tiles: two waves, the second nearly empty)
+  // tiles: instances cut into tile_rows-row pieces, largest first; unless a
+  // caller set their size, smaller batches into smaller pieces, so that the SMs
+  // still share them evenly (12M rows in 64Ki-row tiles are 183 tiles: two
+  // waves, the second nearly empty)
   int64_t all_rows = 0;
   for (auto& I : B.insts) all_rows += I.n_rows;
-  const int64_t tile_rows =
-    std::min(launch.tile_rows, std::max<int64_t>(16384, all_rows / (8 * (int64_t)sms) & ~(int64_t)2047));
+  int64_t tile_rows = launch.tile_rows;
+  if (!launch.exact_tiles)
+    tile_rows = std::min(tile_rows, std::max<int64_t>(16384, all_rows / (8 * (int64_t)sms) & ~(int64_t)2047));
   std::vector<int> order(ninst);
   for (int i = 0; i < ninst; ++i) order[i] = i;
   std::sort(order.begin(), order.end(), [&](int a, int b) { return B.insts[a].n_rows > B.insts[b].n_rows; });
@@ -721,7 +723,7 @@ void Batch::prepare(const std::vector<std::vector<Column>>& keys, int null_polic
   B.smem_bytes = scap_max * stride;
   B.block = launch.block;
   B.stats.block = launch.block;
-  B.stats.tile_rows = launch.tile_rows;
+  B.stats.tile_rows = tile_rows;
   allow_max_smem(Impl::agg_kernel(B.block));
   int bps = 0;
   ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, Impl::agg_kernel(B.block), B.block, B.smem_bytes), "occ");
@@ -963,26 +965,35 @@ int gb_batch_get_stats(const gb_batch* b, gb_batch_stats* out)
   });
 }
 
+static void set_tuning(const gb_batch_rule* rules, int32_t num_rules, const gb_batch_launch* launch, bool exact_tiles)
+{
+  if (num_rules < 0 || (num_rules > 0 && !rules)) throw gb::Error(gb::ERR_LOGIC, "bad batch tuning rules");
+  gb::BatchLaunch L;
+  if (launch) {
+    if (launch->block != 256 && launch->block != 512 && launch->block != 1024)
+      throw gb::Error(gb::ERR_LOGIC, "batch block must be 256, 512 or 1024");
+    if (launch->tile_rows < 1024) throw gb::Error(gb::ERR_LOGIC, "batch tile_rows must be >= 1024");
+    if (launch->smem_bytes < 0) throw gb::Error(gb::ERR_LOGIC, "batch smem_bytes must be >= 0");
+    L.block = launch->block;
+    L.tile_rows = launch->tile_rows;
+    L.smem_bytes = launch->smem_bytes;
+    L.exact_tiles = exact_tiles;
+  }
+  std::vector<gb::BatchRule> v;
+  for (int i = 0; i < num_rules; ++i)
+    v.push_back(gb::BatchRule{rules[i].max_rows, rules[i].max_groups, rules[i].smem_slots,
+                              rules[i].headroom_pct > 0 ? rules[i].headroom_pct / 100.0 : -1.0});
+  gb::set_batch_tuning(v, L);
+}
+
 int gb_batch_set_tuning(const gb_batch_rule* rules, int32_t num_rules, const gb_batch_launch* launch)
 {
-  return guarded([&] {
-    if (num_rules < 0 || (num_rules > 0 && !rules)) throw gb::Error(gb::ERR_LOGIC, "bad batch tuning rules");
-    gb::BatchLaunch L;
-    if (launch) {
-      if (launch->block != 256 && launch->block != 512 && launch->block != 1024)
-        throw gb::Error(gb::ERR_LOGIC, "batch block must be 256, 512 or 1024");
-      if (launch->tile_rows < 1024) throw gb::Error(gb::ERR_LOGIC, "batch tile_rows must be >= 1024");
-      if (launch->smem_bytes < 0) throw gb::Error(gb::ERR_LOGIC, "batch smem_bytes must be >= 0");
-      L.block = launch->block;
-      L.tile_rows = launch->tile_rows;
-      L.smem_bytes = launch->smem_bytes;
-    }
-    std::vector<gb::BatchRule> v;
-    for (int i = 0; i < num_rules; ++i)
-      v.push_back(gb::BatchRule{rules[i].max_rows, rules[i].max_groups, rules[i].smem_slots,
-                                rules[i].headroom_pct > 0 ? rules[i].headroom_pct / 100.0 : -1.0});
-    gb::set_batch_tuning(v, L);
-  });
+  return guarded([&] { set_tuning(rules, num_rules, launch, true); });
+}
+
+int gb_batch_set_default_tuning(const gb_batch_rule* rules, int32_t num_rules, const gb_batch_launch* launch)
+{
+  return guarded([&] { set_tuning(rules, num_rules, launch, false); });
 }
 
 void gb_batch_destroy(gb_batch* b) { delete b; }

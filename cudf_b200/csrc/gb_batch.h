@@ -23,6 +23,7 @@ struct BatchLaunch {
   int block = 512;
   int64_t tile_rows = 65536;
   int smem_bytes = 160 * 1024;
+  bool exact_tiles = false;  // tile_rows was set by a caller: batches of every size take it
 };
 void set_batch_tuning(const std::vector<BatchRule>& rules, const BatchLaunch& launch);
 

@@ -240,7 +240,7 @@ typedef struct gb_batch_stats {
   int32_t kernels_per_run;
   int64_t regrown;          /* instance tables grown after a trial run overflowed */
   int32_t block;            /* threads per CTA of the aggregation launch */
-  int64_t tile_rows;        /* rows per tile of the work queue */
+  int64_t tile_rows;        /* rows per tile of this batch's work queue */
   int64_t ruled_instances;  /* instances a gb_batch_rule sized */
 } gb_batch_stats;
 GB_API int gb_batch_prepare(int32_t num_instances, const gb_column* keys, int32_t num_keys,
@@ -253,9 +253,10 @@ GB_API int gb_batch_get_stats(const gb_batch* batch, gb_batch_stats* out);
 GB_API void gb_batch_destroy(gb_batch* batch);
 
 /* Process-wide tuning of batched launches (no counterpart in libcudf).
- * launch (NULL: defaults 512 threads, 64 Ki-row tiles, 160 KiB tables): the
- * aggregation kernel's threads per CTA (256, 512 or 1024), rows per tile of
- * the work queue, shared-memory bytes of a tile's table.  rules: for each
+ * launch (NULL: defaults 512 threads, 64 Ki-row tiles, fewer rows in batches
+ * of less than 8 tiles per SM, 160 KiB tables): the aggregation kernel's
+ * threads per CTA (256, 512 or 1024), rows per tile of the work queue (taken as
+ * given), shared-memory bytes of a tile's table.  rules: for each
  * instance, the first rule with rows <= max_rows and estimated groups <=
  * max_groups caps its shared table at smem_slots slots (0: global table
  * only; -1: no cap) and takes the shared stage only when groups *
@@ -274,6 +275,11 @@ typedef struct gb_batch_launch {
   int32_t smem_bytes;
 } gb_batch_launch;
 GB_API int gb_batch_set_tuning(const gb_batch_rule* rules, int32_t num_rules, const gb_batch_launch* launch);
+
+/* As gb_batch_set_tuning, for settings that are to be the defaults: tile_rows
+ * is what large batches take, and batches of less than 8 tiles per SM take
+ * fewer rows per tile. */
+GB_API int gb_batch_set_default_tuning(const gb_batch_rule* rules, int32_t num_rules, const gb_batch_launch* launch);
 
 /* Serving loop: continuous batching of groupby queries (no counterpart in
  * libcudf).  gb_server_submit enqueues a query whose columns are resident on
