@@ -44,3 +44,28 @@ def test_wide_records_over_hundreds_to_thousands_of_partitions(columns, groups):
              [agg.sum(), agg.min(), agg.max()]) for c in range(columns)]
     gb, *_ = run_both([cb.Column.from_numpy(key)], reqs, tuning={"force_mode": 2})
     assert gb.stats()["mode"] == 2
+
+
+@pytest.mark.parametrize("two_words", [False, True])
+@pytest.mark.parametrize("nullable", [False, True])
+@pytest.mark.parametrize("hot", [0, 3, 900])
+def test_wide_records_with_hot_keys(hot, nullable, two_words):
+    """96-byte records are read four words at a time: without hot keys, and with keys whose rows are folded per
+    warp first.  The columns' types put their words at every place of a record."""
+    import cudf_b200 as cb
+    from cudf_b200 import aggregation as agg
+    rng = np.random.default_rng(hot + nullable)
+    n = 150_001
+    key = rng.integers(0, 30_000, n)
+    if hot:
+        key = np.where(rng.random(n) < 0.7, rng.integers(0, hot, n), key)
+    keys = [cb.Column.from_numpy(key * 1_000_003)]
+    if two_words:
+        keys.append(cb.Column.from_numpy((key % 11).astype(np.int32)))
+    kinds = [np.int64, np.float64, np.uint64, np.int64, np.float64, np.int64, np.float64, np.int32]
+    if not (nullable or two_words):
+        kinds[-1] = np.int64
+    reqs = [(cb.Column.from_numpy(rng.integers(0, 1000, n).astype(k), rng.random(n) > 0.1 * (j % 3) if nullable else None),
+             [agg.sum(), agg.min(), agg.max(), agg.count()][j % 2:]) for j, k in enumerate(kinds)]
+    gb, *_ = run_both(keys, reqs, tuning={"force_mode": 2})
+    assert gb.stats()["mode"] == 2
