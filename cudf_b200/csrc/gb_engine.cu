@@ -617,8 +617,6 @@ int apply_tuning_rules(Options& o, int64_t rows, int64_t groups, int key_words, 
     if (m & OPT_SMEM_MAX) o.smem_max_groups = r.opt.smem_max_groups;
     if (m & OPT_LOAD) o.load_factor = r.opt.load_factor;
     if (m & OPT_MODE) o.force_mode = r.opt.force_mode;
-    if (m & OPT_SCATTER) o.scatter = r.opt.scatter;
-    if (m & OPT_PASS2) o.pass2 = r.opt.pass2;
     if (m & OPT_PART_FILL) o.part_fill = r.opt.part_fill;
     if (m & OPT_WAGG) o.wagg_pct = r.opt.wagg_pct;
     return (int)i;
@@ -780,11 +778,17 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
   // multiple of the SM count, so that pass 2 ends in whole waves and a tile's
   // runs are no shorter than the tables need; a partition then holds 8 or more
   // of the 2^14 hash buckets, give or take one.  Above that a power of two,
-  // whose partitions hold equally many buckets, at most 8192 (the scatter
-  // keeps 12 B per partition in shared memory); beyond ~85% of that capacity
-  // the shared tables would spill most groups and the global table is faster.
-  int nparts = 0;
+  // whose partitions hold equally many buckets, at most kMaxParts (the scatter
+  // keeps 8 B per partition in shared memory, so kAllParts for some of the
+  // widest records); beyond 80% of that capacity the shared tables would spill
+  // and the global table is faster.  (100M rows, two FLOAT32 sums, 33M groups:
+  // 6.2 ms, global table 16.7, 36M over 8192 partitions 8.8; 30M groups of six
+  // 8-byte accumulators: 9.5 and 35.)
+  RecSpec rec;
+  part_ok = part_ok && record_layout(P, rec);
+  int nparts = 0, max_parts = 0;
   if (part_ok) {
+    max_parts = rec_shape(P.key_words, rec.words, kMaxParts, rec.nmask, dev.smem_optin).threads ? kMaxParts : kAllParts;
     const int64_t sms = dev.sms;
     const int64_t want = std::max<int64_t>(2, (int64_t)std::ceil((double)est / (scap_rec * opt.part_fill)));
     const int64_t tight = (int64_t)std::ceil((double)est / (scap_rec * std::max(opt.part_fill, 0.78)));
@@ -796,9 +800,9 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
     const int64_t whole = (std::max(want, std::min(spread, est / 128 / sms * sms)) + sms - 1) / sms * sms;
     if (want < sms && est < 128 * sms) nparts = (int)std::max(want, est / 128);
     else if (whole <= 2048) nparts = (int)whole;
-    else nparts = (int)std::min<uint64_t>(kMaxParts, next_pow2((uint64_t)tight));
+    else nparts = (int)std::min<uint64_t>(max_parts, next_pow2((uint64_t)tight));
   }
-  const bool part_fits = (double)est <= 0.85 * (double)kMaxParts * sfill2;
+  const bool part_fits = (double)est <= 0.8 * (double)max_parts * scap_rec;
   // VARIANCE/STD look every group up in the global table in their second pass,
   // so partitions only save updates: worth a copy of the rows from a few million
   // of them on, sooner with several accumulators a row than with one or two, and
@@ -818,9 +822,7 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
   else mode = 0;
   if (mode == 1 && scap < 16) mode = 0;
   if (mode == 2 && !(part_ok && opt.partition)) mode = 0;
-  RecSpec rec;
-  if (mode == 2 && !(record_layout(P, rec) && rec_shape(P.key_words, rec.words, nparts, rec.nmask, dev.smem_optin).threads))
-    mode = 0;  // (every record size has a shape up to kMaxParts partitions)
+  if (mode == 2 && !rec_shape(P.key_words, rec.words, nparts, rec.nmask, dev.smem_optin).threads) mode = 0;
 
   if (sampled && mode != 1) {  // only the shared stage does without every row's count
     Options o2 = opt_in;
@@ -1066,7 +1068,7 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
     const int sfill_p = std::max(1, (int)(scap_p * 0.9));
     // groups expected to miss their partition's shared table, plus those of
     // split partitions, go to the global spill table
-    const double expect_spill = std::max(0.0, (double)est - 0.85 * (double)nparts * sfill2);
+    const double expect_spill = std::max(0.0, (double)est - 0.85 * (double)nparts * scap_rec);
     uint64_t spill_cap = next_pow2((uint64_t)std::max<double>(65536.0, 2.0 * expect_spill + 2.0 * (double)nsplit * scap2 +
                                                                               (P.need_second_pass || !deferred ? 2.0 * est : 0.0)));
     // spill list: room for the rows of the groups expected to spill

@@ -9,7 +9,10 @@
 namespace gb {
 
 constexpr int kRecSizes[] = {2, 4, 6, 8, 12};  // 8-byte words of a record
-constexpr int kMaxParts = 8192;                // partitions of one call
+// Partitions of one call: every record size has a launch shape up to kAllParts
+// of them, those of up to 64 bytes (96 without validity masks) up to kMaxParts.
+constexpr int kAllParts = 8192;
+constexpr int kMaxParts = 16384;
 
 // A launch of pass 1: CTAs of `threads` threads, `rows` rows per thread, of
 // which `ctas` share an SM.
