@@ -173,22 +173,15 @@ static uint32_t apply_tuning(const gb_tuning* t, gb::Options& o)
   }
   if (t->groups_hint >= 0) o.groups_hint = t->groups_hint;
   if (t->profile >= 0) o.profile = t->profile;
-  if (t->scatter >= 0) {
-    if (t->scatter > 8) throw gb::Error(gb::ERR_LOGIC, "scatter must be in [0, 8]");
-    o.scatter = t->scatter;
-    m |= gb::OPT_SCATTER;
-  }
+  // scatter, pass2: accepted without effect (see gb_tuning)
+  if (t->scatter > 8) throw gb::Error(gb::ERR_LOGIC, "scatter must be in [0, 8]");
   if (t->part_fill_pct > 0) {
     if (t->part_fill_pct > 95) throw gb::Error(gb::ERR_LOGIC, "part_fill_pct must be in [1, 95]");
     o.part_fill = t->part_fill_pct / 100.0;
     m |= gb::OPT_PART_FILL;
   }
   if (t->wagg_pct >= 0) o.wagg_pct = t->wagg_pct, m |= gb::OPT_WAGG;
-  if (t->pass2 >= 0) {
-    if (t->pass2 > 4) throw gb::Error(gb::ERR_LOGIC, "pass2 must be in [0, 4]");
-    o.pass2 = t->pass2;
-    m |= gb::OPT_PASS2;
-  }
+  if (t->pass2 > 4) throw gb::Error(gb::ERR_LOGIC, "pass2 must be in [0, 4]");
   return m;
 }
 

@@ -78,11 +78,9 @@ struct Options {
   int64_t smem_max_groups = -1;  // use the smem stage when est. groups <= this (-1: derived)
   double load_factor = 0.5;    // global table target load
   int64_t groups_hint = -1;    // caller's group-count estimate (-1: sample)
-  int force_mode = -1;         // -1 auto, 0 global only, 1 smem stage
+  int force_mode = -1;         // -1 auto, 0 global only, 1 smem stage, 2 partitioned
   int profile = 0;             // time kernels with CUDA events
-  int scatter = 7;             // accepted 0-8: earlier launch shapes of partitioned pass 1, which now picks its own
   double part_fill = 0.6;      // partitioned mode: expected groups per partition / shared-table slots (sets the partition count)
-  int pass2 = 1;               // accepted 0-4: earlier forms of partitioned pass 2, which now has one
   int wagg_pct = 125;          // partitioned pass 2: warp-combined updates for partitions above this % of the average rows
   uint32_t set_mask = 0;       // OPT_* bits of the fields a caller set explicitly
   // internal: 0 reads every outcome (group counts, overflow flags, null
@@ -97,7 +95,7 @@ struct Options {
 // Option fields, as bits of Options::set_mask and TuningRule::mask.
 enum OptBits : uint32_t {
   OPT_BLOCK = 1, OPT_BPS = 2, OPT_SMEM = 4, OPT_FILL = 8, OPT_SMEM_MAX = 16, OPT_LOAD = 32,
-  OPT_MODE = 64, OPT_SCATTER = 128, OPT_PASS2 = 256, OPT_PART_FILL = 512, OPT_WAGG = 1024
+  OPT_MODE = 64, OPT_PART_FILL = 512, OPT_WAGG = 1024
 };
 
 // A process-wide tuning rule: for calls with at most max_rows rows and at most
@@ -117,7 +115,7 @@ int apply_tuning_rules(Options& o, int64_t rows, int64_t groups, int key_words, 
 struct Stats {
   int64_t est_groups = 0;
   int64_t capacity = 0;
-  int mode = 0;     // 0 global, 1 smem stage
+  int mode = 0;     // 0 global, 1 smem stage, 2 partitioned
   int retries = 0;
   int kernels = 0;  // kernels launched by this call
   double agg_kernel_ms = 0;  // aggregation kernels (partitioned mode: both passes)

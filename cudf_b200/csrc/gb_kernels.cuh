@@ -66,8 +66,7 @@ __device__ __forceinline__ void update_slot(const Plan& P, uint8_t* slot, int64_
   for (int v = 0; v < P.num_vals; ++v) {
     const ValCol& c = P.vals[v];
     int64_t r = row + c.offset;
-    bool valid = c.bits ? ((c.bits[r] >> c.bit) & 1) : bit_valid(c.mask, r);
-    if (!valid) {
+    if (!bit_valid(c.mask, r)) {
       if (c.nulls_off >= 0) atomicAdd((unsigned int*)(slot + c.nulls_off), 1u);
       continue;
     }

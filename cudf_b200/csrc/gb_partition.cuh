@@ -10,10 +10,10 @@
 //                     in that partition's region.
 //   k_rec_aggregate   pass 2 (gb_record.cuh): one CTA at a time owns a work item
 //                     -- a partition, or a record range of a heavy partition --
-//                     and aggregates it in a shared-memory table; its groups are
-//                     then copied out as dense slots (or merged into a global
-//                     spill table for split partitions and partitions that did
-//                     not fit).
+//                     and aggregates it in a shared-memory table; its groups then
+//                     leave as result rows (or are merged into a global spill
+//                     table: split partitions, partitions that did not fit, and
+//                     VARIANCE/STD, whose second pass looks every group up there).
 //   k_rec_spill       applies the records that did not fit their partition's
 //                     table to the global spill table.
 //
@@ -43,7 +43,6 @@ struct EmitRef {
 // ---- explicit shared-memory operations (32-bit shared-window addresses) ----
 __device__ __forceinline__ void sred_add_u32(uint32_t a, uint32_t v) { asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(a), "r"(v)); }
 __device__ __forceinline__ void sred_add_u64(uint32_t a, uint64_t v) { asm volatile("red.shared.add.u64 [%0], %1;" ::"r"(a), "l"(v)); }
-__device__ __forceinline__ void sred_add_f32(uint32_t a, float v) { asm volatile("red.shared.add.f32 [%0], %1;" ::"r"(a), "f"(v)); }
 __device__ __forceinline__ void sred_add_f64(uint32_t a, double v) { asm volatile("red.shared.add.f64 [%0], %1;" ::"r"(a), "d"(v)); }
 __device__ __forceinline__ void sred_min_u32(uint32_t a, uint32_t v) { asm volatile("red.shared.min.u32 [%0], %1;" ::"r"(a), "r"(v)); }
 __device__ __forceinline__ void sred_max_u32(uint32_t a, uint32_t v) { asm volatile("red.shared.max.u32 [%0], %1;" ::"r"(a), "r"(v)); }
