@@ -686,7 +686,7 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
   // ---- group-count estimate from a key sample ----
   int64_t est;
   const uint32_t* buckets = nullptr;  // rows per hash bucket, in this thread's pinned memory
-  std::vector<uint32_t> even;         // stand-in without a sketch
+  std::vector<uint32_t> flat;         // stand-in without a sketch
   bool exact_buckets = false;  // buckets hold exact row counts (full-pass sketch)
   int64_t nsamp = 0;
   int filled = 0;  // buckets with rows
@@ -762,18 +762,35 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
       sfill = std::max(1, (int)(0.7 * big));
     }
   }
-  int64_t smem_max = opt.smem_max_groups >= 0 ? opt.smem_max_groups : (int64_t)sfill;
-  // partitioned pass 2: as many slots as fit ~220 KB (any count), one more for
-  // the all-ones key
-  const int scap_rec = std::max(0, std::min(220 * 1024, dev.smem_optin - 8192) / (P.slot_bytes + 4) - 1) & ~3;  // with tags
-  const int scap2 = std::max(0, std::min(220 * 1024, dev.smem_optin - 8192) / P.slot_bytes - 1);
-  const int sfill2 = std::max(1, (int)(scap2 * 0.8));
+  // partitioned pass 2 and the shared stage of its plans (closed-form updates):
+  // as many slots as fit ~220 KB (any count, tags beside them), one more for the
+  // all-ones key
+  const int table_bytes = std::min(220 * 1024, dev.smem_optin - 8192);
+  const int scap_rec = std::max(0, table_bytes / (P.slot_bytes + 4) - 1) & ~3;  // with tags
+  const int scap2 = std::max(0, table_bytes / P.slot_bytes - 1);
+  RecSpec rec;
   bool part_ok = !P.has_arg && P.num_vals <= 8 && scap2 >= 256;
   for (int v = 0; v < P.num_vals; ++v) part_ok = part_ok && P.vals[v].basic;
   for (int a = 0; a < P.num_accs; ++a) {
     uint8_t op = P.accs[a].op;
     if (op >= OP_PROD_I64 && op <= OP_PROD_F64) part_ok = false;
   }
+  part_ok = part_ok && record_layout(P, rec);
+  // From 1M rows on the shared stage takes groups up to the fill that the whole
+  // of shared memory stands, where they would otherwise go through partitions or
+  // the global table (FLOAT32 sums in 64 bits widen the slots, and would be the
+  // first to leave it).  Shared stage / else in ms: six FLOAT32 sums, 1800 groups
+  // 1.1M rows 0.21 / 0.54, 2M 0.25 / 0.38, 20M 1.00 / 1.24; two, 4000 groups
+  // (78% fill) 2M 0.21 / 0.34, 20M 0.57 / 0.75.  VARIANCE/STD, 3300 groups (64%)
+  // 2M 0.23 / 0.24, 20M 0.92 / 0.96, 4000 1.06 / 0.96.  Generic updates (ARGMAX),
+  // 2100 groups (52%) 2M 0.23 / 0.24, 20M 1.24 / 1.44; 2500 1.31 / 1.24.
+  const bool own_table = !(opt.set_mask & (OPT_SMEM | OPT_FILL));
+  const int stage_max = (int)(part_ok ? (P.need_second_pass ? 0.7 : 0.85) * scap_rec : 0.55 * scap2);
+  if (own_table && n >= (1 << 20) && est > sfill && est <= stage_max) {
+    scap = scap2;
+    sfill = std::max(1, stage_max);
+  }
+  int64_t smem_max = opt.smem_max_groups >= 0 ? opt.smem_max_groups : (int64_t)sfill;
   // partitions: enough for the wanted table fill.  Up to 2048 they are a
   // multiple of the SM count, so that pass 2 ends in whole waves and a tile's
   // runs are no shorter than the tables need; a partition then holds 8 or more
@@ -784,8 +801,6 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
   // and the global table is faster.  (100M rows, two FLOAT32 sums, 33M groups:
   // 6.2 ms, global table 16.7, 36M over 8192 partitions 8.8; 30M groups of six
   // 8-byte accumulators: 9.5 and 35.)
-  RecSpec rec;
-  part_ok = part_ok && record_layout(P, rec);
   int nparts = 0, max_parts = 0;
   if (part_ok) {
     max_parts = rec_shape(P.key_words, rec.words, kMaxParts, rec.nmask, dev.smem_optin).threads ? kMaxParts : kAllParts;
@@ -811,9 +826,10 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
   // 8M, 500K 0.67 / 0.58; 8M, 4M 1.31 / 1.49; 40M, 20M 9.1 / 10.0.  Four: 1.1M,
   // 50K 0.27 / 0.28; 2M, 5K 0.31 / 0.42; 2M, 200K 0.36 / 0.35; 2M, 1M 0.61 / 0.69;
   // 4M, 5K 0.47 / 0.43; 4M, 200K 0.54 / 0.46; 8M, 4M 2.96 / 2.51.
+  const bool few = est < 128 * (int64_t)dev.sms;  // no partition per SM
   bool part_pays = true;
   if (P.need_second_pass)
-    part_pays = P.num_accs > 2 ? n >= 3500000 || (n >= 2000000 && est >= 128 * (int64_t)dev.sms && n >= 4 * est)
+    part_pays = P.num_accs > 2 ? n >= 3500000 || (n >= 2000000 && !few && n >= 4 * est)
                                : n >= 6000000 && n >= 5 * est;
   int mode;
   if (opt.force_mode >= 0) mode = opt.force_mode;
@@ -838,8 +854,8 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
   bool long_tail = false;
   if (mode == 2) {
     if (!buckets) {  // no sketch (hint given or small input): uniform regions
-      even.assign(kNumBuckets, 1);
-      buckets = even.data();
+      flat.assign(kNumBuckets, 1);
+      buckets = flat.data();
       nsamp = kNumBuckets;
     }
     auto first_bucket = [&](int64_t p) { return (p * kNumBuckets + nparts - 1) / nparts; };  // see part_of
@@ -1160,8 +1176,7 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
 
   // shared stage through k_stage_aggregate: plans whose columns all have
   // closed-form updates and whose groups fit one CTA's ~220 KB table
-  bool raw_stage = mode == 1 && part_ok && opt.block >= 512 && !(opt.set_mask & (OPT_SMEM | OPT_FILL)) &&
-                   est <= (int64_t)(0.7 * sfill2);
+  bool raw_stage = mode == 1 && part_ok && opt.block >= 512 && own_table && est <= (int64_t)(0.85 * scap_rec);
   bool stage_fold = false;
   StageArgs stage;
   std::memset(&stage, 0, sizeof(stage));

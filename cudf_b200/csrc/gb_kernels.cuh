@@ -139,7 +139,6 @@ __global__ void __launch_bounds__(512) k_aggregate(const __grid_constant__ Plan 
     }
   }
   __syncthreads();
-  const uint64_t smask = (uint64_t)scap - 1;
   const int64_t n = P.num_rows;
   int since_check = 0;
   for (int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; row < n;
@@ -154,7 +153,8 @@ __global__ void __launch_bounds__(512) k_aggregate(const __grid_constant__ Plan 
     uint64_t h = hash_key(w0, w1, P.key_words);
     uint8_t* slot = nullptr;
     if (USE_SMEM) {
-      uint64_t i = (h >> 20) & smask;
+      // the middle bits of the hash scaled to the table, of any size
+      uint32_t i = (uint32_t)(((h >> 20 & 0xFFFFFFFFull) * (uint64_t)scap) >> 32);
       if (P.key_words == 1) {
         if (w0 != kEmpty) {
           for (int p = 0; p < 32; ++p) {
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(512) k_aggregate(const __grid_constant__ Plan 
               if (old == kEmpty) { atomicAdd(&s_used, 1u); slot = (uint8_t*)kp; break; }
               if (old == w0) { slot = (uint8_t*)kp; break; }
             }
-            i = (i + 1) & smask;
+            i = i + 1 == (uint32_t)scap ? 0 : i + 1;
           }
         }
       } else {
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(512) k_aggregate(const __grid_constant__ Plan 
             if (old == empty) { atomicAdd(&s_used, 1u); slot = (uint8_t*)kp; break; }
             if (old == want) { slot = (uint8_t*)kp; break; }
           }
-          i = (i + 1) & smask;
+          i = i + 1 == (uint32_t)scap ? 0 : i + 1;
         }
       }
     }
