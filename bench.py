@@ -44,7 +44,7 @@ CPU_SAMPLE_ROWS = N_ROWS
 
 # Kernels whose device time the roofline covers, by engine mode (0 global
 # table, 1 shared-memory stage, 2 hash-partitioned two-pass).
-KERNELS_BY_MODE = {0: "k_aggregate<false>", 1: "k_aggregate<true>",
+KERNELS_BY_MODE = {0: "k_aggregate<false>", 1: "k_stage_aggregate",
                    2: "k_rec_scatter + k_rec_aggregate"}
 # DRAM bytes (read + write) of those kernels per launch, from an ncu capture
 # of a smaller case of the same workload scaled up; the capture command and

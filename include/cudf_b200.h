@@ -129,7 +129,8 @@ GB_API int32_t gb_is_valid_aggregation(int32_t type_id, int32_t kind);
 /* Engine tuning of a handle (no counterpart in libcudf, whose hash path has no
  * tunables: cpp/src/groupby/hash/groupby.cu:64-67,570-572).  Fields < 0 keep
  * the default.  force_mode: -1 auto, 0 global table only, 1 shared-memory stage,
- * 2 hash-partitioned shared-memory aggregation. */
+ * 2 hash-partitioned shared-memory aggregation (a plan it cannot take, or whose
+ * scratch cannot be allocated, runs on the global table). */
 typedef struct gb_tuning {
   int32_t block;            /* threads per CTA of the aggregation kernel */
   int32_t blocks_per_sm;    /* CTAs per SM (0 = occupancy limit) */
