@@ -1,7 +1,8 @@
 """Per-size-bucket autotuner for the engine's launch parameters.
 
 The engine's kernels have tunables (mode thresholds, shared-memory table size
-and fill, global-table load factor, the partitions' table fill).  The best values depend on the call's size: rows and distinct groups.  This module
+and fill, global-table load factor, the partitions' table fill).  The best
+values depend on the call's size: rows and distinct groups.  This module
 times candidate settings on synthetic inputs of each (rows, groups) bucket
 with CUDA events, keeps the fastest, and installs the result as process-wide
 rules (``gb_set_tuning_rules``): a call takes the first rule whose bucket

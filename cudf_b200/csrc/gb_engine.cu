@@ -1315,16 +1315,19 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
     if (deferred) {
       // an overflow anywhere (a table, a region, the result rows, a spill
       // list): redo the call with checks after every stage, or, where only a
-      // sample had sized it, from the count of every row
+      // sample or the caller's estimate had sized it, from the count of every row
       const bool again = host[1] || chost[1] || (mode == 2 && (host[5] || host[13])) ||
                          (raw_stage && host[13]);
       if (again) {
         R.release();
         Options o2 = opt_in;
-        o2.sync_checks = !sampled;
+        o2.sync_checks = !sampled && opt.groups_hint < 0;
         o2.full_sketch = 1;
+        o2.groups_hint = -1;
         S.clear();
-        return aggregate_call(keys, null_policy, reqs, stream, alloc, o2, stats, state);
+        Result again_r = aggregate_call(keys, null_policy, reqs, stream, alloc, o2, stats, state);
+        if (stats) ++stats->retries;
+        return again_r;
       }
       const int64_t dn = mode == 2 ? (int64_t)(host[10] | ((uint64_t)host[11] << 32)) : 0;
       G_n = (int64_t)chost[2];

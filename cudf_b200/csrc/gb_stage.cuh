@@ -120,7 +120,9 @@ __global__ void __launch_bounds__(1024, 1) k_stage_aggregate(const __grid_consta
     __syncwarp();
     apply_columns<R, MAXV, FOLD>(S, nc, P.rows_off, sa, vb, x);
   }
-  __syncthreads();
+  // the list overflowed: the call is redone, and its merges would search a full
+  // table for each group
+  if (__syncthreads_or(threadIdx.x == 0 && *(volatile unsigned int*)(A.counters + 13))) return;
   // the other copies into the first
   const RecTable first = table_of(0);
   for (int i = A.slots + threadIdx.x; i < total; i += NT) {
@@ -134,7 +136,10 @@ __global__ void __launch_bounds__(1024, 1) k_stage_aggregate(const __grid_consta
   __syncthreads();
   for (int i = threadIdx.x; i < A.slots; i += NT) {
     const uint8_t* s = slots + (size_t)i * stride;
-    if (slot_occupied(P, s, false)) merge_slot(P, G, s, &s_new);
+    if (slot_occupied(P, s, false)) {
+      if (*(volatile unsigned int*)(G.counters + 1)) break;  // the global table is full: as above
+      merge_slot(P, G, s, &s_new);
+    }
   }
   if (KW == 1 && threadIdx.x == 0) {
     const uint8_t* s = slot_at(total);
@@ -150,7 +155,8 @@ static __global__ void __launch_bounds__(256) k_stage_spill(const __grid_constan
   __shared__ unsigned int s_new;
   if (threadIdx.x == 0) s_new = 0;
   __syncthreads();
-  const unsigned cnt = min(*(volatile unsigned int*)(A.counters + 12), A.spill_cap);
+  unsigned cnt = min(*(volatile unsigned int*)(A.counters + 12), A.spill_cap);
+  if (*(volatile unsigned int*)(A.counters + 13) || *(volatile unsigned int*)(G.counters + 1)) cnt = 0;  // redone anyway
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
     const int64_t r = A.spill_rows[i];
     uint64_t w0, w1;

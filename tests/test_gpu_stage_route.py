@@ -36,6 +36,20 @@ def test_stage_route(plan, n, groups, mode):
     assert gb.stats()["mode"] == mode
 
 
+@pytest.mark.parametrize("plan", ["2 sums", "sums, argmax", "var"])
+@pytest.mark.parametrize("groups,hint,redone", [(2_000, 2_000, False), (40_000, 2_000, True), (300_000, 20_000, True)])
+def test_a_caller_s_estimate_far_too_low_is_dropped(plan, groups, hint, redone):
+    """A right estimate holds; one that the tables overflow on is replaced by the count of every row."""
+    import cudf_b200 as cb
+    rng = np.random.default_rng(groups)
+    n = 1_100_000
+    key = rng.integers(0, groups, n) * 1_000_003
+    gb, uk, *_ = run_both([cb.Column.from_numpy(key)], _requests(plan, rng, n), tuning={"groups_hint": hint})
+    st = gb.stats()
+    assert st["retries"] == int(redone)
+    assert abs(st["est_groups"] - uk.num_rows()) < 0.08 * uk.num_rows()
+
+
 @pytest.mark.parametrize("plan", ["2 sums", "sums, argmax"])
 @pytest.mark.parametrize("key", ["i64", "two words"])
 def test_generic_stage_tables_of_any_size(plan, key):
