@@ -1370,14 +1370,19 @@ Result aggregate(const std::vector<Column>& keys, int null_policy, const std::ve
                  cudaStream_t stream, const Allocator& alloc, const Options& opt, Stats* stats)
 {
   CallState state;
+  auto settle = [&] {  // the thread's next call writes its pinned staging again
+    if (state.staged) cudaStreamSynchronize(stream);
+  };
   try {
     return aggregate_call(keys, null_policy, reqs, stream, alloc, opt, stats, state);
   } catch (const Error& e) {
-    // the thread's next call writes its pinned staging again
-    if (state.staged) cudaStreamSynchronize(stream);
+    settle();
     // rows as records can take up to about twice the columns' bytes: without
     // room for them the global table, which needs no copy of the rows
     if (e.code != ERR_ALLOC || !state.partitioned) throw;
+  } catch (...) {
+    settle();
+    throw;
   }
   Options o2 = opt;
   o2.partition = 0;
