@@ -775,7 +775,6 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
     uint8_t op = P.accs[a].op;
     if (op >= OP_PROD_I64 && op <= OP_PROD_F64) part_ok = false;
   }
-  part_ok = part_ok && record_layout(P, rec);
   // From 1M rows on the shared stage takes groups up to the fill that the whole
   // of shared memory stands, where they would otherwise go through partitions or
   // the global table (FLOAT32 sums in 64 bits widen the slots, and would be the
@@ -802,7 +801,9 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
   // 6.2 ms, global table 16.7, 36M over 8192 partitions 8.8; 30M groups of six
   // 8-byte accumulators: 9.5 and 35.)
   int nparts = 0, max_parts = 0;
-  if (part_ok) {
+  const bool may_part = part_ok && opt.partition && (opt.force_mode == 2 || (opt.force_mode < 0 && n >= (1 << 20))) &&
+                        record_layout(P, rec);
+  if (may_part) {
     max_parts = rec_shape(P.key_words, rec.words, kMaxParts, rec.nmask, dev.smem_optin).threads ? kMaxParts : kAllParts;
     const int64_t sms = dev.sms;
     const int64_t want = std::max<int64_t>(2, (int64_t)std::ceil((double)est / (scap_rec * opt.part_fill)));
@@ -834,10 +835,10 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
   int mode;
   if (opt.force_mode >= 0) mode = opt.force_mode;
   else if (scap >= 64 && est <= smem_max) mode = 1;
-  else if (part_ok && part_fits && part_pays && n >= (1 << 20) && est > smem_max) mode = 2;
+  else if (may_part && part_fits && part_pays && est > smem_max) mode = 2;
   else mode = 0;
   if (mode == 1 && scap < 16) mode = 0;
-  if (mode == 2 && !(part_ok && opt.partition)) mode = 0;
+  if (mode == 2 && !may_part) mode = 0;
   if (mode == 2 && !rec_shape(P.key_words, rec.words, nparts, rec.nmask, dev.smem_optin).threads) mode = 0;
 
   if (sampled && mode != 1) {  // only the shared stage does without every row's count
