@@ -442,12 +442,22 @@ inline size_t sketch_smem() { return ((size_t(1) << kHllBits) + (size_t(1) << kB
 // chunks > 0: only that many runs of 128 rows, one from each of `chunks` equal
 // strata at a scrambled place (so that no period of the data can hide groups).
 // skip (optional): a device flag; set, the kernel leaves at once.
+// runs: [0] rows looked at (one warp load in 32), [1] those whose key is that of
+// the row before them: sorted or clustered keys, whose rows meet in a warp.
 static __global__ void __launch_bounds__(512) k_sketch(const __grid_constant__ Plan P, unsigned int* hll,
-                                                       unsigned int* buckets, int64_t chunks, const unsigned int* skip)
+                                                       unsigned int* buckets, int64_t chunks, const unsigned int* skip,
+                                                       unsigned int* runs)
 {
   constexpr int NT = 512;
   constexpr int SR = 4;
   if (skip && *skip) return;
+  unsigned looked = 0, same = 0, step_no = 0;
+  auto neighbours = [&](uint32_t key, bool live) {  // every lane of the warp
+    const uint32_t before = __shfl_up_sync(0xFFFFFFFFu, key, 1);
+    const bool counts = live && (threadIdx.x & 31) > 0;
+    looked += counts;
+    same += counts && before == key;
+  };
   extern __shared__ unsigned int sk[];
   unsigned int* reg = sk;
   unsigned int* bk = sk + (1 << kHllBits);
@@ -472,6 +482,8 @@ static __global__ void __launch_bounds__(512) k_sketch(const __grid_constant__ P
       uint64_t k[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) k[j] = __ldg(kd + row + j * stride);
+      if ((step_no++ & 7) == 0 && (row | 31) + 3 * stride < n)  // the whole warp is here
+        neighbours((uint32_t)(k[0] ^ (k[0] >> 32)), true);
 #pragma unroll
       for (int j = 0; j < 4; ++j) add(fmix64(k[j]));
     }
@@ -515,9 +527,18 @@ static __global__ void __launch_bounds__(512) k_sketch(const __grid_constant__ P
       for (int j = 0; j < SR; ++j) live[j] = w0 + lane + 32 * j < n;
       pack_rows<2, SR>(P, w0 + lane, k0, k1, live);
 #pragma unroll
-      for (int j = 0; j < SR; ++j)
-        if (live[j]) add(hash_key(k0[j], k1[j], P.key_words));
+      for (int j = 0; j < SR; ++j) {
+        const uint64_t h = hash_key(k0[j], k1[j], P.key_words);
+        if (j == 0 && (step_no++ & 7) == 0) neighbours((uint32_t)h, live[0]);
+        if (live[j]) add(h);
+      }
     }
+  }
+  looked = __reduce_add_sync(0xFFFFFFFFu, looked);
+  same = __reduce_add_sync(0xFFFFFFFFu, same);
+  if ((threadIdx.x & 31) == 0 && looked) {
+    atomicAdd(runs, looked);
+    atomicAdd(runs + 1, same);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < (1 << kHllBits); i += NT)

@@ -1,0 +1,24 @@
+"""Keys in sorted order: rows of one key meet in a warp, and are folded there
+before they update a table."""
+import numpy as np
+import pytest
+
+from parity import run_both
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("two_words", [False, True])
+@pytest.mark.parametrize("n,groups,mode", [(70_001, 40, None), (200_000, 900, 1), (1_100_000, 2_000, 1),
+                                           (1_500_000, 20_000, 2), (1_500_000, 400_000, 2), (8_400_000, 30, 1)])
+def test_sorted_keys(n, groups, mode, two_words):
+    import cudf_b200 as cb
+    from cudf_b200 import aggregation as agg
+    rng = np.random.default_rng(n + groups)
+    key = np.sort(rng.integers(0, groups, n)) - 3  # an all-ones key among them
+    keys = [cb.Column.from_numpy(key)] + ([cb.Column.from_numpy((key % 2).astype(np.int32), rng.random(n) > 0.001)] if two_words else [])
+    reqs = [(cb.Column.from_numpy(rng.integers(-10**9, 10**9, n), rng.random(n) > 0.1), [agg.sum(), agg.min(), agg.count()]),
+            (cb.Column.from_numpy(rng.normal(size=n).astype(np.float32)), [agg.sum(), agg.max()])]
+    gb, *_ = run_both(keys, reqs, include_null_keys=two_words)
+    if mode is not None and not two_words:
+        assert gb.stats()["mode"] == mode
