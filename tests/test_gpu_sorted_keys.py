@@ -1,5 +1,5 @@
-"""Keys in sorted order: rows of one key meet in a warp, and are folded there
-before they update a table."""
+"""Keys in sorted order, and hot keys: rows of one key meet in a warp, and are
+folded there before they update a table."""
 import numpy as np
 import pytest
 
@@ -22,3 +22,17 @@ def test_sorted_keys(n, groups, mode, two_words):
     gb, *_ = run_both(keys, reqs, include_null_keys=two_words)
     if mode is not None and not two_words:
         assert gb.stats()["mode"] == mode
+
+
+@pytest.mark.parametrize("n,groups,mode", [(1_500_000, 60_000, 2), (6_000_000, 16_000, 2)])
+@pytest.mark.parametrize("share", [0.06, 0.7])
+def test_a_hot_key_among_many(n, groups, mode, share):
+    import cudf_b200 as cb
+    from cudf_b200 import aggregation as agg
+    rng = np.random.default_rng(n)
+    key = rng.integers(0, groups, n) * 1_000_003
+    key[rng.random(n) < share] = 77
+    reqs = [(cb.Column.from_numpy(rng.integers(-10**9, 10**9, n)), [agg.sum(), agg.max()]),
+            (cb.Column.from_numpy(rng.normal(size=n), rng.random(n) > 0.1), [agg.sum(), agg.min()])]
+    gb, *_ = run_both([cb.Column.from_numpy(key)], reqs)
+    assert gb.stats()["mode"] == mode
