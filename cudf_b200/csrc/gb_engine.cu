@@ -791,9 +791,11 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
   // (78% fill) 2M 0.21 / 0.34, 20M 0.57 / 0.75.  VARIANCE/STD, 3300 groups (64%)
   // 2M 0.23 / 0.24, 20M 0.92 / 0.96, 4000 1.06 / 0.96.  Generic updates (ARGMAX),
   // 2100 groups (52%) 2M 0.23 / 0.24, 20M 1.24 / 1.44; 2500 1.31 / 1.24.
+  // With a hot key or in sorted order from 64Ki rows on: those queue on the
+  // global table's slots (880K rows, 1700 groups, 70% of them one's: 2.7 ms).
   const bool own_table = !(opt.set_mask & (OPT_SMEM | OPT_FILL));
   const int stage_max = (int)(part_ok ? (P.need_second_pass ? 0.7 : 0.85) * scap_rec : 0.55 * scap2);
-  if (own_table && n >= (1 << 20) && est > sfill && est <= stage_max) {
+  if (own_table && (n >= (1 << 20) || hot || clustered) && est > sfill && est <= stage_max) {
     scap = scap2;
     sfill = std::max(1, stage_max);
   }
