@@ -37,3 +37,15 @@ def test_a_hot_key_among_many(n, groups, mode, share):
     gb, *_ = run_both([cb.Column.from_numpy(key)], reqs)
     if n > 1_000_000 or share > 0.1:
         assert gb.stats()["mode"] == mode
+
+
+@pytest.mark.parametrize("n,groups", [(300_000, 30), (1_500_000, 65), (1_500_000, 250)])
+def test_sorted_keys_with_many_accumulators(n, groups):
+    import cudf_b200 as cb
+    from cudf_b200 import aggregation as agg
+    rng = np.random.default_rng(groups)
+    keys = [cb.Column.from_numpy(np.sort(rng.integers(0, groups, n)))]
+    reqs = [(cb.Column.from_numpy(rng.integers(-10**9, 10**9, n) if i % 2 else rng.normal(size=n)), [agg.sum(), agg.min(), agg.max()])
+            for i in range(7)]
+    gb, *_ = run_both(keys, reqs)
+    assert gb.stats()["mode"] == 1
