@@ -1056,11 +1056,17 @@ Result aggregate_call(const std::vector<Column>& keys, int null_policy, const st
       // soonest, in whole waves over the SMs, an item's table and merges counted
       // as 2Ki rows (few partitions have few groups each).  In items of 32Ki rows
       // 2M rows of 5500 groups were 42 whole partitions: six FLOAT32 sums 0.45
-      // ms, now 0.30; 4M rows of 7000 groups 0.58, now 0.41.
-      const bool even = exact_buckets && nparts < dev.sms && nrows < 65536 * (int64_t)dev.sms;
+      // ms, now 0.30; 4M rows of 7000 groups 0.58, now 0.41.  Under a long tail
+      // the partitions are far from equal and so are their pieces, up to half
+      // as long again: three or more to an SM even out (7M Zipf rows of 16K
+      // groups, 12 accumulators: 0.80, whole partitions 1.05, 32Ki-row items
+      // 0.87; 9.5M rows 1.04 against 0.98 with 32Ki, so the line is lower).
+      const bool even =
+        exact_buckets && nparts < dev.sms && nrows < (long_tail ? 57344 : 65536) * (int64_t)dev.sms;
       if (even) {
         int64_t best = INT64_MAX;
         for (int64_t k = 1; k <= 16; ++k) {
+          if (long_tail && nparts * k < 3 * dev.sms) continue;
           const int64_t end = (nparts * k + dev.sms - 1) / dev.sms * (share / k + 2048);
           if (end < best) best = end, chunk = std::max<int64_t>(64, share / k);
         }

@@ -49,3 +49,16 @@ def test_sorted_keys_with_many_accumulators(n, groups):
             for i in range(7)]
     gb, *_ = run_both(keys, reqs)
     assert gb.stats()["mode"] == 1
+
+
+@pytest.mark.parametrize("n,groups", [(1_200_000, 8_000), (2_000_000, 16_000), (7_000_001, 16_000)])
+def test_long_tailed_keys_in_few_partitions(n, groups):
+    import cudf_b200 as cb
+    from cudf_b200 import aggregation as agg
+    rng = np.random.default_rng(n + groups)
+    top = (groups + 1.0) ** -0.1
+    key = np.minimum(((1 - rng.random(n) * (1 - top)) ** -10.0 - 1).astype(np.int64), groups - 1) * 1_000_003
+    reqs = [(cb.Column.from_numpy(rng.integers(-10**9, 10**9, n)), [agg.sum(), agg.min()]),
+            (cb.Column.from_numpy(rng.normal(size=n), rng.random(n) > 0.1), [agg.sum(), agg.max()])]
+    gb, *_ = run_both([cb.Column.from_numpy(key)], reqs)
+    assert gb.stats()["mode"] == 2
